@@ -147,12 +147,12 @@ struct OpSphereMask {        // rho := 0 where x^2+y^2+z^2 >= rad2, all cells of
 // over the base blocks in list order and, inside a block, k, j, i; the two
 // kernels below keep that order, so the moments -- and with them the whole
 // isolated-boundary solve -- are bit-identical to a serial evaluation:
-// k_moment_terms evaluates each cell's 25 terms in parallel (the reference's
-// expressions, left to right), k_moments_ordered adds them in cell order,
-// one lane per moment, with the loads running ahead of the dependent adds.
+// k_moment_terms evaluates each cell's terms in parallel (the reference's
+// expressions, left to right) into one array per moment, k_moments_ordered
+// adds each array in cell order.
 constexpr int kMomentTerms = 25;
 __global__ void k_moment_terms(const double *R, const double *x0, const double *h0, int n, int G, int64_t V,
-                               int nbase, int lmax, double *T /* [nbase n^3][25] */) {
+                               int nbase, int lmax, double *T /* [25][nbase n^3] */) {
     pdl_enter();
     const int64_t ncell = (int64_t)nbase * n * n * n;
     const double h = h0[0], dv = h * h * h;
@@ -168,40 +168,38 @@ __global__ void k_moment_terms(const double *R, const double *x0, const double *
         double ri = 1 / rr, rci = 1 / rc;
         double cost = z * ri, sint = rc * ri, cosp = x * rci, sinp = y * rci;
         double rhodv = R[(int64_t)b * V + cidx(G, i, j, k)] * dv;
-        double *t = T + c * kMomentTerms;
-        t[0] = rhodv;
-        t[1] = rhodv * rr * cost;
-        t[2] = rhodv * rr * sint * cosp;
-        t[3] = rhodv * rr * sint * sinp;
-        t[4] = rhodv * r2 * (3 * (cost * cost) - 1);
-        t[5] = rhodv * r2 * sint * cost * cosp;
-        t[6] = rhodv * r2 * sint * cost * sinp;
-        t[7] = rhodv * r2 * (sint * sint) * ((cosp * cosp) - (sinp * sinp));
-        t[8] = rhodv * r2 * (sint * sint) * 2 * sinp * cosp;
-        t[9] = rhodv * r3 * cost * (5 * (cost * cost) - 3);
-        t[10] = rhodv * r3 * sint * (5 * (cost * cost) - 1) * cosp;
-        t[11] = rhodv * r3 * sint * (5 * (cost * cost) - 1) * sinp;
-        t[12] = rhodv * r3 * cost * (sint * sint) * ((cosp * cosp) - (sinp * sinp));
-        t[13] = rhodv * r3 * cost * (sint * sint) * 2 * sinp * cosp;
-        t[14] = rhodv * r3 * (sint * sint * sint) * cosp * ((cosp * cosp) - 3 * (sinp * sinp));
-        t[15] = rhodv * r3 * (sint * sint * sint) * sinp * (3 * (cosp * cosp) - (sinp * sinp));
+        auto t = [&](int m) -> double & { return T[(int64_t)m * ncell + c]; };
+        t(0) = rhodv;
+        t(1) = rhodv * rr * cost;
+        t(2) = rhodv * rr * sint * cosp;
+        t(3) = rhodv * rr * sint * sinp;
+        t(4) = rhodv * r2 * (3 * (cost * cost) - 1);
+        t(5) = rhodv * r2 * sint * cost * cosp;
+        t(6) = rhodv * r2 * sint * cost * sinp;
+        t(7) = rhodv * r2 * (sint * sint) * ((cosp * cosp) - (sinp * sinp));
+        t(8) = rhodv * r2 * (sint * sint) * 2 * sinp * cosp;
+        t(9) = rhodv * r3 * cost * (5 * (cost * cost) - 3);
+        t(10) = rhodv * r3 * sint * (5 * (cost * cost) - 1) * cosp;
+        t(11) = rhodv * r3 * sint * (5 * (cost * cost) - 1) * sinp;
+        t(12) = rhodv * r3 * cost * (sint * sint) * ((cosp * cosp) - (sinp * sinp));
+        t(13) = rhodv * r3 * cost * (sint * sint) * 2 * sinp * cosp;
+        t(14) = rhodv * r3 * (sint * sint * sint) * cosp * ((cosp * cosp) - 3 * (sinp * sinp));
+        t(15) = rhodv * r3 * (sint * sint * sint) * sinp * (3 * (cosp * cosp) - (sinp * sinp));
         if (lmax >= 4) {
             double r4 = r2 * r2, c2 = cost * cost, s2 = sint * sint;
             double cos2p = (cosp * cosp) - (sinp * sinp), sin2p = 2 * sinp * cosp;
             double cos3p = cosp * ((cosp * cosp) - 3 * (sinp * sinp));
             double sin3p = sinp * (3 * (cosp * cosp) - (sinp * sinp));
             double cos4p = cos2p * cos2p - sin2p * sin2p, sin4p = 2 * sin2p * cos2p;
-            t[16] = rhodv * r4 * (35 * (c2 * c2) - 30 * c2 + 3);
-            t[17] = rhodv * r4 * sint * cost * (7 * c2 - 3) * cosp;
-            t[18] = rhodv * r4 * sint * cost * (7 * c2 - 3) * sinp;
-            t[19] = rhodv * r4 * s2 * (7 * c2 - 1) * cos2p;
-            t[20] = rhodv * r4 * s2 * (7 * c2 - 1) * sin2p;
-            t[21] = rhodv * r4 * s2 * sint * cost * cos3p;
-            t[22] = rhodv * r4 * s2 * sint * cost * sin3p;
-            t[23] = rhodv * r4 * (s2 * s2) * cos4p;
-            t[24] = rhodv * r4 * (s2 * s2) * sin4p;
-        } else {
-            for (int m = 16; m < kMomentTerms; m++) t[m] = 0.0;
+            t(16) = rhodv * r4 * (35 * (c2 * c2) - 30 * c2 + 3);
+            t(17) = rhodv * r4 * sint * cost * (7 * c2 - 3) * cosp;
+            t(18) = rhodv * r4 * sint * cost * (7 * c2 - 3) * sinp;
+            t(19) = rhodv * r4 * s2 * (7 * c2 - 1) * cos2p;
+            t(20) = rhodv * r4 * s2 * (7 * c2 - 1) * sin2p;
+            t(21) = rhodv * r4 * s2 * sint * cost * cos3p;
+            t(22) = rhodv * r4 * s2 * sint * cost * sin3p;
+            t(23) = rhodv * r4 * (s2 * s2) * cos4p;
+            t(24) = rhodv * r4 * (s2 * s2) * sin4p;
         }
     }
 }
@@ -247,26 +245,75 @@ __device__ __forceinline__ double zmirror_factor(int m) {
                               (1u << 18) | (1u << 21) | (1u << 22);
     return ((kOdd >> m) & 1u) ? 0.0 : 2.0;
 }
-// one warp; lane m < 25 sums term m over the cells in order
+// CTA m < nterm sums moment m over the cells in order: eight warps stage the
+// next chunk of terms into shared memory, each its own stretch of it, while
+// thread 0 adds the current one (the sequence of roundings of a
+// single-thread loop).  Terms equal to zero are left out, as adding +-0
+// changes no running sum that started at +0 (it never becomes -0): the mask
+// zeroes 48% of a cubic box's cells.  A stretch is padded with +0 to whole
+// groups.  Bound by the chain of dependent FP64 adds (8 cycles each).  On the
+// 64^3 base cells of a sphere, 25 moments: 0.71 ms; one warp, a lane per
+// moment and 16 loads ahead of its adds, was bound by the loads' latency
+// (37 ns a term): 9.87 ms.
 // mode 0: the sphere's normalisations; 1: the same times the z-mirror
 // factors; 2: the z-periodic cylinders' a00 = (sum of term 0) / zlen / pi2
-// (cyl_zperiodic.F90:197) in mom[0]
-__global__ void __launch_bounds__(32) k_moments_ordered(const double *__restrict__ T, int64_t ncell, double *mom,
-                                                         int mode, double zlen, double pi2) {
+// (cyl_zperiodic.F90:197) in mom[0].  Moments from nterm on (the l = 4 terms
+// with lmax = 3) have no terms: their sum is 0.
+constexpr int kMomentWarps = 8, kMomentStretch = 256, kMomentThreads = 32 * (kMomentWarps + 1);
+__global__ void __launch_bounds__(kMomentThreads) k_moments_ordered(const double *__restrict__ T, int64_t ncell,
+                                                                    int nterm, double *mom, int mode, double zlen,
+                                                                    double pi2) {
     pdl_enter();
-    const int m = threadIdx.x;
-    if (m >= kMomentTerms) return;
-    constexpr int U = 16;   // loads issued ahead of the dependent adds
+    constexpr int U = 16, CH = kMomentWarps * kMomentStretch;   // adds per group, terms per chunk
+    __shared__ __align__(16) double tm[2][kMomentWarps][kMomentStretch];
+    __shared__ int cnt[2][kMomentWarps];
+    const int m = blockIdx.x, tid = threadIdx.x, w = (tid >> 5) - 1, lane = tid & 31;
     double a = 0.0;
-    int64_t c = 0;
-    for (; c + U <= ncell; c += U) {
-        double t[U];
+    if (m < nterm) {   // CTA-uniform
+        const double *Tm = T + (int64_t)m * ncell;
+        const int64_t nch = (ncell + CH - 1) / CH;
+        auto stage = [&](int64_t c) {   // warp w of the staging warps
+            const int64_t o = c * CH + w * kMomentStretch;
+            double v[kMomentStretch / 32];
 #pragma unroll
-        for (int u = 0; u < U; u++) t[u] = T[(c + u) * kMomentTerms + m];
+            for (int r = 0; r < kMomentStretch / 32; r++) v[r] = o + r * 32 + lane < ncell ? Tm[o + r * 32 + lane] : 0.0;
+            double *q = tm[c & 1][w];
+            int k = 0;
 #pragma unroll
-        for (int u = 0; u < U; u++) a = a + t[u];
+            for (int r = 0; r < kMomentStretch / 32; r++) {
+                const unsigned keep = __ballot_sync(0xffffffffu, v[r] != 0.0);
+                if (v[r] != 0.0) q[k + __popc(keep & ((1u << lane) - 1))] = v[r];
+                k += __popc(keep);
+            }
+            const int full = (k + U - 1) / U * U;
+            if (lane < full - k) q[k + lane] = 0.0;
+            if (lane == 0) cnt[c & 1][w] = full;
+        };
+        if (w >= 0 && nch > 0) stage(0);
+        __syncthreads();
+        for (int64_t c = 0; c < nch; c++) {
+            if (w >= 0) {
+                if (c + 1 < nch) stage(c + 1);
+            } else if (tid == 0) {
+                for (int s = 0; s < kMomentWarps; s++) {
+                    const double2 *q = reinterpret_cast<const double2 *>(tm[c & 1][s]);
+                    const int n = cnt[c & 1][s];
+                    double2 v[U / 2];
+                    for (int e = 0; e < n; e += U) {
+#pragma unroll
+                        for (int u = 0; u < U / 2; u++) v[u] = q[e / 2 + u];
+#pragma unroll
+                        for (int u = 0; u < U / 2; u++) {
+                            a = a + v[u].x;
+                            a = a + v[u].y;
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+        }
     }
-    for (; c < ncell; c++) a = a + T[c * kMomentTerms + m];
+    if (tid != 0) return;
     if (mode == 2) {
         if (m == 0) mom[0] = a / zlen / pi2;
         return;

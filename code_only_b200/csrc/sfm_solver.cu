@@ -1690,7 +1690,8 @@ public:
         const int64_t ncell = (int64_t)cnt(0) * n * n * n;
         launch_pdl(k_moment_terms, (unsigned)std::min<int64_t>((ncell + 255) / 256, (int64_t)nSM * 8), 256, 0, SRC0,
                    d_x0, d_h0, n, Gf[0], Vf[0], cnt(0), P.lmax, d_part);
-        launch_pdl(k_moments_ordered, 1, 32, 0, d_part, ncell, d_mom, zm ? 1 : 0, 1.0, 1.0);
+        launch_pdl(k_moments_ordered, kMomentTerms, kMomentThreads, 0, d_part, ncell, P.lmax >= 4 ? kMomentTerms : 16,
+                   d_mom, zm ? 1 : 0, 1.0, 1.0);
         launches += 2;
         int GT = n + 2;
         run(OpSphereGhost{PSI0, d_tfL, d_mom, d_x0, d_h0, d_level, n, Gf[0], Vf[0], P.lmax}, tfLOff[H.nlev] * GT * GT);
@@ -1717,7 +1718,7 @@ public:
         launch_pdl(k_moment_terms, (unsigned)std::min<int64_t>((ncell + 255) / 256, (int64_t)nSM * 8), 256, 0, SRC0,
                    d_x0, d_h0, n, Gf[0], Vf[0], cnt(0), P.lmax, d_part);
         const double pi2 = 2.0 * (4.0 * std::atan(1.0));   // Pi2 (parameter.F90:14-15)
-        launch_pdl(k_moments_ordered, 1, 32, 0, d_part, ncell, d_mom, 2, zlen, pi2);
+        launch_pdl(k_moments_ordered, 1, kMomentThreads, 0, d_part, ncell, 1, d_mom, 2, zlen, pi2);
         launches += 2;
         int GT = n + 2;
         run(OpCylGhost{PSI0, d_tfL, d_cyllog, d_mom, n, Gf[0], Vf[0]}, tfLOff[H.nlev] * GT * GT);
