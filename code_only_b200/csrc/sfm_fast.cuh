@@ -1211,10 +1211,25 @@ __global__ void __launch_bounds__(256) k_resid_tiled(TO *__restrict__ res, const
     }
 }
 
+// cell (i, j, k) of block b into the planes it lies on
+template <class T, int N>
+__device__ __forceinline__ void faces_put(T *out, int64_t b, int i, int j, int k, T v) {
+    constexpr int NN = N * N;
+    T *o = out + b * (6 * NN);
+    if (i == 0) o[k * N + j] = v;
+    if (i == N - 1) o[NN + k * N + j] = v;
+    if (j == 0) o[2 * NN + k * N + i] = v;
+    if (j == N - 1) o[3 * NN + k * N + i] = v;
+    if (k == 0) o[4 * NN + j * N + i] = v;
+    if (k == N - 1) o[5 * NN + j * N + i] = v;
+}
+
 // ---------------------------------------------------------------------------
 // prolongation of listed blocks: fine level (N) interior from the same block
 // one fmg level coarser (N/2 + 2 cells with ghosts), tricubic staged as
-// interp_tricubic stages bufx / bufxy (interpolation.F90:98-217), or trilinear
+// interp_tricubic stages bufx / bufxy (interpolation.F90:98-217), or
+// trilinear.  add: the value is added to uf (fmg_addint, fmg.F90:942-946)
+// instead of stored; faces: also left in the boundary planes (sfm_faces.cuh)
 // ---------------------------------------------------------------------------
 // blocks per CTA of k_interp_tiled: at least 512 fine cells per CTA, and
 // four 8^3 blocks (the per-CTA weights, load and three barriers amortised
@@ -1223,7 +1238,8 @@ template <int N>
 __host__ __device__ constexpr int interp_bpc() { return N == 8 ? 4 : (N * N * N >= 512 ? 1 : 512 / (N * N * N)); }
 template <class T, int N>
 __global__ void __launch_bounds__(256) k_interp_tiled(T *__restrict__ uf, const T *__restrict__ uc,
-                                                      const int32_t *__restrict__ blocks, int nblk, int cubic) {
+                                                      const int32_t *__restrict__ blocks, int nblk, int cubic,
+                                                      int add, T *__restrict__ faces) {
     pdl_enter();
     constexpr int NC = N / 2, GC = NC + 2, GF = N + 2;
     constexpr int VC = GC * GC * GC, VF = GF * GF * GF;
@@ -1251,11 +1267,17 @@ __global__ void __launch_bounds__(256) k_interp_tiled(T *__restrict__ uf, const 
         sc[t] = uc[(int64_t)sb[q] * VC + (t - q * VC)];
     }
     __syncthreads();
+    auto put = [&](int q, int i, int j, int k, T v) {
+        T *o = uf + (int64_t)sb[q] * VF + cidx(GF, i, j, k);
+        if (add) v = *o + v;
+        *o = v;
+        if (faces) faces_put<T, N>(faces, sb[q], i, j, k, v);
+    };
     if (!(cubic && NC + 2 >= 4)) {
         for (int t = threadIdx.x; t < nq * NF; t += blockDim.x) {
             const int q = t / NF, r = t - q * NF;
             const int i = r % N, j = (r / N) % N, k = r / (N * N);
-            uf[(int64_t)sb[q] * VF + cidx(GF, i, j, k)] = trilinear_cell(sc + q * VC, GC, i, j, k, 0, 0, 0);
+            put(q, i, j, k, trilinear_cell(sc + q * VC, GC, i, j, k, 0, 0, 0));
         }
         return;
     }
@@ -1288,7 +1310,7 @@ __global__ void __launch_bounds__(256) k_interp_tiled(T *__restrict__ uf, const 
         const T *w = cwt[k];
         const T *bq = bxy + q * BXY;
         auto Y = [&](int kc) { return bq[((kc + 1) * N + j) * N + i]; };
-        uf[(int64_t)sb[q] * VF + cidx(GF, i, j, k)] = w[0] * Y(c[0]) + w[1] * Y(c[1]) + w[2] * Y(c[2]) + w[3] * Y(c[3]);
+        put(q, i, j, k, w[0] * Y(c[0]) + w[1] * Y(c[1]) + w[2] * Y(c[2]) + w[3] * Y(c[3]));
     }
 }
 

@@ -47,6 +47,7 @@
 #include "sfm_kernels_misc.cuh"
 #include "sfm_mg.cuh"
 #include "sfm_fast.cuh"
+#include "sfm_faces.cuh"
 #include "sfm_noalloc.cuh"
 #include "sfm_adjoint.cuh"
 #include "sfm_tune.h"
@@ -330,6 +331,13 @@ public:
                                            // cell of the boundary faces (d_tfL order), from the host's libm
     bool zperiodic() const { return P.bc == SFM_BC_CYL_ZPERIODIC || P.bc == SFM_BC_MASK_ZPERIODIC; }
     int nLeaves = 0, nReflux = 0, nSlots = 0;
+    // plane exchange of the sweeps (sfm_faces.cuh): per fmg level the boundary
+    // planes (two buffers of [6 nb][n^2] in turn) and the coarse-fine ghost planes
+    bool facesOk = false;                  // every margin of a coarse-fine face has a plain source
+    int32_t *d_fsrc = nullptr, *d_child = nullptr;
+    CFItem *d_cf = nullptr;
+    std::vector<T *> faceBuf[2], cfBuf;
+    std::vector<int> facePar;              // buffer holding U[f]'s planes, -1: neither
     std::vector<int> leafList;
 
     // fields: inner precision T at every fmg level, FP64 outer fields at level 0
@@ -346,7 +354,8 @@ public:
     int *d_err = nullptr;                  // set by a device wait that gave up
     uint32_t waitPolls = kWaitPolls;       // poll limit of the smoother's stage waits (tests lower it)
     int nSM = 148;
-    int bulkGrid[5][4][4] = {};            // persistent CTAs of k_relax_bulk<T, N, NT, SW>, by log2(N), NT, SW
+    int bulkGrid[5][4] = {};               // persistent CTAs of k_relax_bulk, by log2(N), SW
+    int faceGrid[5][4][4] = {};            // of k_relax_faces, by log2(N), CTA size, SW
     double *d_mom = nullptr, *d_part = nullptr, *d_psum = nullptr;
     int *d_mgit = nullptr;
     // base grid
@@ -640,13 +649,13 @@ public:
                 const bool fused = kind == 1;
                 if (fused && sizeof(T) != 4) continue;
                 float best = std::numeric_limits<float>::max();
-                int pick = n >= 16 ? 512 : 256;
+                int pick = relax_nt(n, fused);
                 for (int nt : kRelaxNT) {
+                    if (!faces_at(f)) break;   // k_relax_bulk has one CTA size
                     tune.set(kKnobRelaxThreads, (int)sizeof(T), n, -1, kind, nt);
                     const float t = time_min([&] {
                         for (int ipass = 1; ipass <= (fused ? 1 : 2); ipass++)
-                            relax_launch(U[f], RHS[f], d_leaves, nLeaves, d_rslot, rbuf[f], f, ipass, d_max,
-                                         fused ? 1 : 0);
+                            relax_faces_launch(U[f], RHS[f], f, ipass, d_max, fused ? 1 : 0, false);
                     }, reps);
                     if (t < best) { best = t; pick = nt; }
                 }
@@ -915,6 +924,7 @@ public:
                         }
                 gCnt[L][sel + 1] = (int)((int64_t)gitems.size() - gOff[L][sel + 1]);
             }
+        faces_tables(refl);
         d_level = mem.upload(std::vector<int32_t>(H.level.begin(), H.level.end()));
         d_parent = mem.upload(std::vector<int32_t>(H.parent.begin(), H.parent.end()));
         d_oct = mem.upload(H.oct);
@@ -970,6 +980,12 @@ public:
         for (int f = 0; f <= FMax; f++) {
             U.push_back(fieldT(f)); RES.push_back(fieldT(f)); RHS.push_back(fieldT(f)); RHO.push_back(fieldT(f));
             rbuf.push_back(mem.alloc<double>((size_t)std::max(nSlots, 1) * nf[f] * nf[f]));
+            const size_t nn = facesOk && face_edge(nf[f]) ? (size_t)nf[f] * nf[f] : 0;
+            for (auto &b : faceBuf) b.push_back(nn ? mem.alloc<T>((size_t)nb * 6 * nn) : nullptr);
+            cfBuf.push_back(nn ? mem.alloc<T>((size_t)(nReflux + 1) * nn) : nullptr);   // and a plane of zeros
+            if (nn && cfBuf.back() && cudaMemset(cfBuf.back() + (size_t)nReflux * nn, 0, nn * sizeof(T)) != cudaSuccess)
+                mem.err = cudaErrorUnknown;
+            facePar.push_back(-1);
         }
         RUF = fieldT(FMax);
         SRC0 = fieldD(0); PSI0 = fieldD(0); PHI0 = fieldD(0); RES0d = fieldD(0);
@@ -1036,6 +1052,100 @@ public:
             return mem.err == cudaErrorMemoryAllocation ? SFM_ENOMEM : SFM_ECUDA;
         }
         return SFM_OK;
+    }
+
+    // Tables of the plane exchange: the source of every leaf face's ghost
+    // plane, and per coarse-fine face (in refl's order) the sources of the
+    // coarse plane's margin: the coarse block's transverse ghost cells, which
+    // the passes fill across same-level faces (highest dimension first for the
+    // edge between both).  facesOk is left false -- the ghost passes serve the
+    // sweeps -- where a margin has another source: a coarse-fine ghost of the
+    // coarse block, or a refined block whose child there is refined again.
+    // Proper nesting over all 26 neighbours excludes both; the links alone
+    // only guarantee the faces.  The z-mirror box, whose mirror plane is a
+    // ghost plane of its own kind, keeps the passes too.
+    void faces_tables(const std::vector<RefluxItem> &refl) {
+        if (P.bc == SFM_BC_ZMIRROR) return;
+        std::vector<int32_t> src(6 * (size_t)H.nb, kFaceZero);
+        for (int b = 0; b < H.nb; b++) {
+            if (H.skip[b]) continue;
+            for (int f = 0; f < 6; f++)
+                if (H.sameLev[6 * b + f] && !H.skip[H.nbrGid[6 * b + f]]) src[6 * b + f] = 6 * H.nbrGid[6 * b + f] + (f ^ 1);
+        }
+        bool ok = true;
+        // block across face f of block b: >= 0, kFaceZero at the physical boundary
+        auto across = [&](int b, int f) -> int {
+            if (H.sameLev[6 * b + f]) return H.nbrGid[6 * b + f];
+            if (!H.touch[6 * b + f]) ok = false;   // a coarser neighbour
+            return kFaceZero;
+        };
+        std::vector<CFItem> items;
+        for (size_t k = 0; k < refl.size(); k++) {
+            const RefluxItem &r = refl[k];
+            const int fc = (1 - r.lr) + 2 * r.dir;
+            int c = -1;
+            if (r.fine >= 0) c = H.nbrGid[6 * r.fine + r.lr + 2 * r.dir];
+            CFItem it{};
+            it.fine = r.fine; it.coarse = c; it.slot = r.slot;
+            it.dir = r.dir; it.lr = r.lr; it.oa = r.oa; it.ob = r.ob;
+            if (H.skip[c] || H.skip[r.fine]) ok = false;
+            const int da = tra(r.dir), db = trb(r.dir), fa = it.oa + 2 * da, fb = it.ob + 2 * db;
+            const int A = across(c, fa), B = across(c, fb), AB = B == kFaceZero ? kFaceZero : across(B, fa);
+            // a refined margin block: its children on the coarse block's side must be leaves
+            auto source = [&](int D, bool fixA, bool fixB) -> int32_t {
+                if (D < 0 || !H.skip[D]) return D;
+                for (int x = 0; x < 2; x++)
+                    for (int y = 0; y < 2; y++) {
+                        if ((fixA && x != 1 - it.oa) || (fixB && y != 1 - it.ob)) continue;
+                        int o[3];
+                        put3(r.dir, fc & 1, x, y, o[0], o[1], o[2]);
+                        const int ch = H.child[8 * D + o[0] + 2 * o[1] + 4 * o[2]];
+                        if (ch < 0 || H.skip[ch]) ok = false;
+                    }
+                return -2 - D;
+            };
+            it.ma = source(A, true, false);
+            it.mb = source(B, false, true);
+            it.mab = source(AB, true, true);
+            src[6 * r.fine + r.lr + 2 * r.dir] = face_cf((int)k);
+            items.push_back(it);
+        }
+        if (!ok) return;
+        facesOk = true;
+        d_fsrc = mem.upload(src);
+        d_child = mem.upload(std::vector<int32_t>(H.child.begin(), H.child.end()));
+        d_cf = mem.upload(items);
+    }
+    // block edges the plane exchange serves: those of the bulk-copy sweeps
+    static bool face_edge(int n) {
+        bool ok = false;
+        SFM_WITH_N(n, ok = bulk_ok<N>(), ok = false)
+        return ok;
+    }
+    bool faces_at(int f) const { return facesOk && !serialRelax && face_edge(nf[f]); }
+    FaceArgs<T> face_args(int f, bool zero) const {
+        const int p = facePar[f] < 0 ? 0 : facePar[f];
+        return FaceArgs<T>{faceBuf[p][f], faceBuf[1 - p][f], cfBuf[f], cfBuf[f] + (size_t)nReflux * nf[f] * nf[f], d_fsrc,
+                           zero ? 1 : 0};
+    }
+    // planes of u valid, coarse-fine ghosts and corrected fluxes of the sweep or residual that follows
+    void faces_flux(int f, const T *u) {
+        if (facePar[f] < 0) {
+            facePar[f] = 0;
+            SFM_WITH_N(nf[f],
+                       (launch_pdl(k_faces_of<T, N>, (unsigned)std::min<int64_t>(((int64_t)nLeaves * 6 * N * N + 255) / 256,
+                                                                                  (int64_t)nSM * 16),
+                                   256, 0, u, faceBuf[0][f], (const int32_t *)d_leaves, nLeaves),
+                        ++launches),
+                       (void)0)
+        }
+        if (nReflux > 0)
+            SFM_WITH_N(nf[f],
+                       (launch_pdl(k_cf_reflux<T, N>, (unsigned)(((int64_t)nReflux * (N / 2) * (N / 2) + 127) / 128), 128, 0,
+                                   u, (const T *)faceBuf[facePar[f]][f], cfBuf[f], rbuf[f], (const CFItem *)d_cf, nReflux,
+                                   (const int32_t *)d_child, (const double *)d_h0, (const int32_t *)d_level, f),
+                        ++launches),
+                       (void)0)
     }
 
     // -----------------------------------------------------------------
@@ -1236,7 +1346,7 @@ public:
     }
     // fmg_poisson_flux (fmg_poisson.F90:53-124)
     template <class TT>
-    void poisson_flux(int f, TT *u, bool bf0) {
+    void poisson_flux(int f, TT *u, bool bf0, bool withReflux = true) {
         if (FmgLevel_fill0 != f) {
             converge_c2p(f, u);
             fmg_boundary_u(f, u);
@@ -1245,21 +1355,35 @@ public:
             fmg_boundary_u(f, u);
         }
         FmgLevel_fill0 = Undef;
-        reflux(f, u);
+        if (withReflux) reflux(f, u);
     }
 
     // -----------------------------------------------------------------
     // fmg level operations on the inner fields
-    void relax(int f, T *u, T *rhs, bool bf0, int slot) {   // fmg_poisson_relax
-        cudaMemsetAsync(d_max + slot, 0, sizeof(unsigned long long), st_);
+    // fmg_poisson_relax.  slot: where |resh2| is folded (slot 0 is read by the
+    // stopping rule and starts at zero; the others are not read).  keepGhosts:
+    // the ghost layer as it is before the last colour is read later, so the
+    // ghost passes run before it even where the planes serve the sweep.
+    void relax(int f, T *u, T *rhs, bool bf0, int slot, bool keepGhosts) {
+        if (slot == 0) cudaMemsetAsync(d_max + slot, 0, sizeof(unsigned long long), st_);
         // the mixed schedule may sweep both colours in one launch (one ghost
         // refresh per sweep instead of one per colour)
-        const bool fused = fused_at(f);
-        for (int ipass = 1; ipass <= (fused ? 1 : 2); ipass++) {
-            poisson_flux(f, u, bf0);
+        const bool fused = fused_at(f), planes = faces_at(f) && u == U[f];
+        const int npass = fused ? 1 : 2;
+        for (int ipass = 1; ipass <= npass; ipass++) {
+            const bool zero = FmgLevel_fill0 == f;
+            if (!planes || (keepGhosts && ipass == npass)) poisson_flux(f, u, bf0, !planes);
+            FmgLevel_fill0 = Undef;
+            if (planes && !zero) faces_flux(f, u);
             const bool prof = f == 0 && profNext < (int)profEv.size() / 2;
             if (prof) prof_mark(2 * profNext);
-            relax_launch(u, rhs, d_leaves, nLeaves, d_rslot, rbuf[f], f, ipass, d_max + slot, fused ? local_sweeps() : 0);
+            if (planes) {
+                relax_faces_launch(u, rhs, f, ipass, d_max + slot, fused ? local_sweeps() : 0, zero);
+                facePar[f] = facePar[f] < 0 ? 1 : 1 - facePar[f];
+            } else {
+                relax_launch(u, rhs, d_leaves, nLeaves, d_rslot, rbuf[f], f, ipass, d_max + slot,
+                             fused ? local_sweeps() : 0);
+            }
             if (prof) prof_mark(2 * profNext++ + 1);
         }
     }
@@ -1288,35 +1412,48 @@ public:
     static constexpr int kRelaxNT[4] = {256, 288, 512, 544};
     template <int NT>
     static constexpr int nt_index() { return NT == 256 ? 0 : (NT == 288 ? 1 : (NT == 512 ? 2 : 3)); }
-    template <int N, int NT, int SW>
-    int bulk_grid() {
+    // resident CTAs of a persistent kernel over the whole GPU (its dynamic
+    // shared memory opted in whatever the size: static and dynamic together
+    // may pass 48 KB)
+    template <class K>
+    int resident(K kern, int nt, int smem) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        int per = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, nt, smem) != cudaSuccess || per < 1) {
+            cudaGetLastError();
+            per = 1;
+        }
+        return nSM * per;
+    }
+    template <int N>
+    static constexpr int log2_edge() { return N >= 16 ? 4 : (N >= 8 ? 3 : 2); }   // capped
+    template <int N, int SW>
+    int bulk_grid() {   // k_relax_bulk
         if constexpr (!bulk_ok<N>()) {
             return 0;
         } else {
-            constexpr int li = N >= 16 ? 4 : (N >= 8 ? 3 : 2);   // log2(N), capped
-            constexpr int ti = nt_index<NT>();
-            if (!bulkGrid[li][ti][SW]) {
-                const int smem = BulkPlan<T, N>::SMEM;
-                // opt in whatever the size: static and dynamic shared memory together may pass 48 KB
-                cudaFuncSetAttribute(k_relax_bulk<T, N, NT, SW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-                int per = 0;
-                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_relax_bulk<T, N, NT, SW>, NT, smem) !=
-                        cudaSuccess ||
-                    per < 1) {
-                    cudaGetLastError();
-                    per = 1;
-                }
-                bulkGrid[li][ti][SW] = nSM * per;
-            }
-            return bulkGrid[li][ti][SW];
+            int &g = bulkGrid[log2_edge<N>()][SW];
+            if (!g) g = resident(k_relax_bulk<T, N, relax_bulk_threads<N>(), SW>, relax_bulk_threads<N>(), BulkPlan<T, N>::SMEM);
+            return g;
+        }
+    }
+    template <int N, int NT, int SW>
+    int face_grid() {   // k_relax_faces
+        if constexpr (!bulk_ok<N>()) {
+            return 0;
+        } else {
+            int &g = faceGrid[log2_edge<N>()][nt_index<NT>()][SW];
+            if (!g) g = resident(k_relax_faces<T, N, NT, SW>, NT, FacePlan<T, N>::SMEM);
+            return g;
         }
     }
     template <int N, int SW>
     void bulk_grids_of() {
-        (void)bulk_grid<N, 256, SW>();
-        (void)bulk_grid<N, 288, SW>();
-        (void)bulk_grid<N, 512, SW>();
-        (void)bulk_grid<N, 544, SW>();
+        (void)bulk_grid<N, SW>();
+        (void)face_grid<N, 256, SW>();
+        (void)face_grid<N, 288, SW>();
+        (void)face_grid<N, 512, SW>();
+        (void)face_grid<N, 544, SW>();
     }
     template <int N>
     void bulk_grids() {   // every variant a solve may launch
@@ -1327,39 +1464,64 @@ public:
             bulk_grids_of<N, 3>();
         }
     }
-    template <int N, int NT, int SW>
+    template <int N, int SW>
     void relax_bulk_launch(T *u, const T *rhs, const int32_t *blocks, int nblk, const int32_t *rslot, const double *rb,
                            int f, int ipass, unsigned long long *out) {
-        launch_pdl(k_relax_bulk<T, N, NT, SW>,
-                   (unsigned)std::min((nblk + Tile<N>::BPC - 1) / Tile<N>::BPC, bulk_grid<N, NT, SW>()), NT,
-                   BulkPlan<T, N>::SMEM, u, rhs, blocks, nblk, d_h0, d_level, rslot, rb, f, ipass, out, d_err, waitPolls);
+        launch_pdl(k_relax_bulk<T, N, relax_bulk_threads<N>(), SW>,
+                   (unsigned)std::min((nblk + Tile<N>::BPC - 1) / Tile<N>::BPC, bulk_grid<N, SW>()),
+                   relax_bulk_threads<N>(), BulkPlan<T, N>::SMEM, u, rhs, blocks, nblk, d_h0, d_level, rslot, rb, f, ipass,
+                   out, d_err, waitPolls);
+    }
+    template <int N, int NT, int SW>
+    void relax_faces_nt(T *u, const T *rhs, int f, int ipass, unsigned long long *out, bool zero) {
+        launch_pdl(k_relax_faces<T, N, NT, SW>,
+                   (unsigned)std::min((nLeaves + Tile<N>::BPC - 1) / Tile<N>::BPC, face_grid<N, NT, SW>()), NT,
+                   FacePlan<T, N>::SMEM, u, rhs, (const int32_t *)d_leaves, nLeaves, (const double *)d_h0,
+                   (const int32_t *)d_level, (const int32_t *)d_rslot, (const double *)rbuf[f], face_args(f, zero), f,
+                   ipass, out, d_err, waitPolls);
     }
     template <int N, int SW>
-    void relax_bulk_nt(int nt, T *u, const T *rhs, const int32_t *blocks, int nblk, const int32_t *rslot,
-                       const double *rb, int f, int ipass, unsigned long long *out) {
-        switch (nt) {
-            case 288: relax_bulk_launch<N, 288, SW>(u, rhs, blocks, nblk, rslot, rb, f, ipass, out); break;
-            case 512: relax_bulk_launch<N, 512, SW>(u, rhs, blocks, nblk, rslot, rb, f, ipass, out); break;
-            case 544: relax_bulk_launch<N, 544, SW>(u, rhs, blocks, nblk, rslot, rb, f, ipass, out); break;
-            default: relax_bulk_launch<N, 256, SW>(u, rhs, blocks, nblk, rslot, rb, f, ipass, out); break;
+    void relax_faces_sw(T *u, const T *rhs, int f, int ipass, unsigned long long *out, bool zero) {
+        switch (relax_nt(N, SW > 0)) {
+            case 256: relax_faces_nt<N, 256, SW>(u, rhs, f, ipass, out, zero); break;
+            case 512: relax_faces_nt<N, 512, SW>(u, rhs, f, ipass, out, zero); break;
+            case 544: relax_faces_nt<N, 544, SW>(u, rhs, f, ipass, out, zero); break;
+            default: relax_faces_nt<N, 288, SW>(u, rhs, f, ipass, out, zero); break;
         }
     }
-    // CTA size of the bulk smoother at block edge n, two-launch sweep (tune
-    // key kind -1) or fused sweeps (kind 1)
+    // the sweep over all leaves with planes: one colour, or sw > 0 full sweeps
+    void relax_faces_launch(T *u, const T *rhs, int f, int ipass, unsigned long long *out, int sw, bool zero) {
+        auto go = [&](auto edge) {
+            constexpr int N = decltype(edge)::value;
+            if constexpr (bulk_ok<N>()) {
+                if constexpr (sizeof(T) == 4) {   // the FP64 path always runs the reference's two colour launches
+                    if (sw == 1) return relax_faces_sw<N, 1>(u, rhs, f, ipass, out, zero);
+                    if (sw == 2) return relax_faces_sw<N, 2>(u, rhs, f, ipass, out, zero);
+                    if (sw == 3) return relax_faces_sw<N, 3>(u, rhs, f, ipass, out, zero);
+                }
+                relax_faces_sw<N, 0>(u, rhs, f, ipass, out, zero);
+            }
+        };
+        if (nLeaves <= 0) return;
+        SFM_WITH_N(nf[f], go(std::integral_constant<int, N>{}), (void)0)
+        ++launches;
+    }
+    // CTA size of k_relax_faces at block edge n, two-launch sweep (tune key
+    // kind -1) or fused sweeps (kind 1); by default the consumer warps divide
+    // a tile's cell pairs evenly (8 warps for 256 pairs, 16 for 2048)
     int relax_nt(int n, bool fused) const {
-        return tune.get(kKnobRelaxThreads, (int)sizeof(T), n, -1, fused ? 1 : -1, n >= 16 ? 512 : 256);
+        return tune.get(kKnobRelaxThreads, (int)sizeof(T), n, -1, fused ? 1 : -1, n >= 16 ? 544 : 288);
     }
     template <int N>
     void relax_dispatch(T *u, const T *rhs, const int32_t *blocks, int nblk, const int32_t *rslot, const double *rb,
                         int f, int ipass, unsigned long long *out, int sw) {
         if constexpr (bulk_ok<N>()) {
-            const int nt = relax_nt(N, sw > 0);
             if constexpr (sizeof(T) == 4) {   // the FP64 path always runs the reference's two colour launches
-                if (sw == 1) return relax_bulk_nt<N, 1>(nt, u, rhs, blocks, nblk, rslot, rb, f, ipass, out);
-                if (sw == 2) return relax_bulk_nt<N, 2>(nt, u, rhs, blocks, nblk, rslot, rb, f, ipass, out);
-                if (sw == 3) return relax_bulk_nt<N, 3>(nt, u, rhs, blocks, nblk, rslot, rb, f, ipass, out);
+                if (sw == 1) return relax_bulk_launch<N, 1>(u, rhs, blocks, nblk, rslot, rb, f, ipass, out);
+                if (sw == 2) return relax_bulk_launch<N, 2>(u, rhs, blocks, nblk, rslot, rb, f, ipass, out);
+                if (sw == 3) return relax_bulk_launch<N, 3>(u, rhs, blocks, nblk, rslot, rb, f, ipass, out);
             }
-            relax_bulk_nt<N, 0>(nt, u, rhs, blocks, nblk, rslot, rb, f, ipass, out);
+            relax_bulk_launch<N, 0>(u, rhs, blocks, nblk, rslot, rb, f, ipass, out);
         } else {
             launch_pdl(k_relax_tiled<T, N>, (unsigned)std::min((nblk + Tile<N>::BPC - 1) / Tile<N>::BPC, persistGrid),
                        256, 0, u, rhs, blocks, nblk, d_h0, d_level, rslot, rb, f, ipass, sizeof(T) == 4 ? sw : 0,
@@ -1499,8 +1661,10 @@ public:
     template <class TA, class TD>
     void add(int f, TA *a, const TD *d) { runB(OpAdd<TA, TD>{a, d, d_leaves, Vf[f]}, nLeaves); }
 
-    // fmg_interp (fmg.F90:786-822)
-    void fmg_interp(int f, T *uf, T *uc, bool cubic) {
+    // fmg_interp (fmg.F90:786-822) of U[f + 1] into uf, or added to it
+    // (fmg_addint, fmg.F90:942-946; uf must be U[f]).  The planes of U[f] are
+    // left with it where the sweeps exchange planes.
+    void fmg_interp(int f, T *uf, T *uc, bool cubic, bool addTo = false) {
         int lc = f + 1;
         converge_c2p(lc, uc, cubic);
         fmg_boundary_u(lc, uc);
@@ -1508,22 +1672,51 @@ public:
         boundary_extrap(lc, uc);
         fmg_boundary_u(lc, uc);
         const int n = nf[f];
+        T *planes = nullptr;
+        if (uf == U[f] && faces_at(f)) {
+            facePar[f] = 0;
+            planes = faceBuf[0][f];
+        }
         SFM_WITH_N(n,
                    (launch_pdl(k_interp_tiled<T, N>, (unsigned)((nLeaves + interp_bpc<N>() - 1) / interp_bpc<N>()), 256, 0, uf,
-                               uc, d_leaves, nLeaves, cubic ? 1 : 0),
+                               uc, d_leaves, nLeaves, cubic ? 1 : 0, addTo ? 1 : 0, planes),
                     ++launches),
                    run(OpInterp<T>{uf, uc, d_leaves, n, Gf[f], Gf[lc], Vf[f], Vf[lc], cubic ? 1 : 0},
                        (int64_t)nLeaves * n * n * n))
         boundary_fill0(lc, uc);
-        boundary_fill0(f, uf);
+        if (!addTo) boundary_fill0(f, uf);   // an addend's zero ghosts change nothing
         fmg_boundary_u(lc, uc);
         fmg_boundary_u(f, uf);
     }
 
+    // the descent step of fmg_lin: residual of level v restricted to the next
+    // level's right-hand side, that level's correction zeroed
+    void resid_rstrct_fill0(int v) {
+        if (!faces_at(v)) {
+            resid(v, RES[v], U[v], RHS[v], true);
+            fmg_rstrct(v + 1, RHS[v + 1], RES[v]);
+            fill0(v + 1, U[v + 1]);
+        } else {
+            faces_flux(v, U[v]);
+            auto go = [&](auto edge) {
+                constexpr int N = decltype(edge)::value;
+                if constexpr (bulk_ok<N>()) {
+                    launch_pdl(k_resid_faces<T, N>, (unsigned)((nLeaves + resid_faces_bpc<N>() - 1) / resid_faces_bpc<N>()),
+                               256, 0, (const T *)U[v], (const T *)RHS[v], RHS[v + 1], U[v + 1],
+                               (const int32_t *)d_leaves, nLeaves, (const double *)d_h0, (const int32_t *)d_level,
+                               (const int32_t *)d_rslot, (const double *)rbuf[v], face_args(v, false), v);
+                    ++launches;
+                }
+            };
+            SFM_WITH_N(nf[v], go(std::integral_constant<int, N>{}), (void)0)
+        }
+        FmgLevel_fill0 = v + 1;
+    }
     // fmg_lin (fmg.F90:270-377)
     void fmg_lin() {
         nvtxRangePushA("sfm fmg_lin");
         const int FMax = H.FMax;
+        for (int &p : facePar) p = -1;
         for (int f = 1; f <= FMax; f++) fmg_rstrct(f, RHO[f], RHO[f - 1]);
         fill0(FMax, U[FMax]);
         vmg_fas(false);
@@ -1533,17 +1726,25 @@ public:
             const int ncycle = sched(kKnobFmgCycles, 2), nsweep = sched(kKnobFmgSweeps, 2);
             for (int jc = 1; jc <= ncycle; jc++) {
                 for (int v = f; v <= FMax - 1; v++) {
-                    for (int q = 0; q < nsweep; q++) relax(v, U[v], RHS[v], true, 0);
-                    resid(v, RES[v], U[v], RHS[v], true);
-                    fmg_rstrct(v + 1, RHS[v + 1], RES[v]);
-                    fill0(v + 1, U[v + 1]);
-                    FmgLevel_fill0 = v + 1;
+                    for (int q = 0; q < nsweep; q++) relax(v, U[v], RHS[v], true, 4, false);
+                    resid_rstrct_fill0(v);
                 }
                 vmg_fas(true);
                 for (int v = FMax - 1; v >= f; v--) {
-                    fmg_interp(v, RES[v], U[v + 1], false);   // fmg_addint
-                    add(v, U[v], RES[v]);
-                    for (int q = 0; q < nsweep; q++) relax(v, U[v], RHS[v], true, 0);
+                    if (faces_at(v)) {
+                        fmg_interp(v, U[v], U[v + 1], false, true);   // fmg_addint
+                    } else {
+                        fmg_interp(v, RES[v], U[v + 1], false);
+                        add(v, U[v], RES[v]);
+                    }
+                    for (int q = 0; q < nsweep; q++) {
+                        // the level's last sweep: the cubic restriction of the
+                        // next fmg level (level 0: the caller) reads the ghost
+                        // layer it leaves, and level 0's maximum is the one
+                        // the stopping rule takes
+                        const bool last = jc == ncycle && v == f && q == nsweep - 1;
+                        relax(v, U[v], RHS[v], true, last && v == 0 ? 0 : 4, last);
+                    }
                 }
             }
         }
