@@ -46,6 +46,7 @@
 #include "sfm_device.cuh"
 #include "sfm_kernels_misc.cuh"
 #include "sfm_mg.cuh"
+#include "sfm_mgs.cuh"
 #include "sfm_fast.cuh"
 #include "sfm_faces.cuh"
 #include "sfm_noalloc.cuh"
@@ -692,7 +693,7 @@ public:
             }
         }
         // base-grid launch: one CTA or a cluster (same cells, same expressions)
-        if (useSerialMg) {
+        if (useSerialMg && mgsTop == 0) {
             struct Cand { int nct, wide; };
             std::vector<Cand> cands = {{1, 16}};
             for (int nct : {2, 4, 8, 16})
@@ -1046,6 +1047,7 @@ public:
             mg.SRC = mem.alloc<double>(V0); mg.PSI = mem.alloc<double>(V0);
             zeroList.push_back({mg.SRC, V0 * sizeof(double)});
             zeroList.push_back({mg.PSI, V0 * sizeof(double)});
+            mgs_init();
         }
         if (mem.err != cudaSuccess) {
             last_error = cudaGetErrorString(mem.err);
@@ -1828,11 +1830,94 @@ public:
             return;
         }
         const int F = H.FMax;
+        if (mgsTop > 0) {   // gather, cycle and scatter in one launch
+            mgs_with([&](auto kern, int ctas, size_t smem) {
+                const MgsArgs a{d_baseIdx, H.ngb[0], nf[F], Gf[F], Vf[F], mg.hbase, sched(kKnobBaseCorr, 10)};
+                mgs_launch(kern, ctas, smem, u, (const T *)rhs, a);
+            });
+            return;
+        }
         int64_t N3 = (int64_t)NBc * NBc * NBc;
         run(OpMgGather<T>{mg.SRC, mg.PSI, rhs, u, d_baseIdx, H.ngb[0], H.ngb[1], nf[F], Gf[F], NBc, Vf[F]}, N3);
         mg_launch(tune.get(kKnobBaseCtas, (int)sizeof(T), NBc, -1, -1, 1),
                   tune.get(kKnobBaseWide, (int)sizeof(T), NBc, -1, -1, 16));
         run(OpMgScatter<T>{u, mg.PSI, d_baseIdx, H.ngb[0], H.ngb[1], nf[F], Gf[F], NBc, Vf[F]}, N3);
+    }
+    // k_mgs_cycle for this base grid: go(kernel, CTAs of the cluster, shared bytes)
+    int mgsTop = 0, mgsMode = 0;   // log2 of the base grid's edge (0: k_mg_cycle), MgMode
+    template <int TOP, int C, class F>
+    void mgs_mode(F &&go) {
+        constexpr size_t smem = (size_t)Mgs<TOP, C, 0>::total() * sizeof(double);
+        switch (mgsMode) {
+            case kMgPeriodic: go(k_mgs_cycle<T, TOP, C, kMgPeriodic>, C, smem); break;
+            case kMgIsolated: go(k_mgs_cycle<T, TOP, C, kMgIsolated>, C, smem); break;
+            case kMgZMirror: go(k_mgs_cycle<T, TOP, C, kMgZMirror>, C, smem); break;
+            default: go(k_mgs_cycle<T, TOP, C, kMgZPeriodic>, C, smem); break;
+        }
+    }
+    template <class F>
+    void mgs_with(F &&go) {
+        switch (mgsTop) {
+            case 1: mgs_mode<1, 1>(go); break;
+            case 2: mgs_mode<2, 1>(go); break;
+            case 3: mgs_mode<3, 1>(go); break;
+            case 4: mgs_mode<4, 1>(go); break;
+            default: mgs_mode<5, 8>(go); break;
+        }
+    }
+    template <class K>
+    void mgs_launch(K kern, int ctas, size_t smem, T *u, const T *rhs, const MgsArgs &a) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[2];
+        mgs_config(cfg, at, ctas, smem);
+        cudaLaunchKernelEx(&cfg, kern, u, rhs, a);
+        ++launches;
+    }
+    void mgs_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int ctas, size_t smem) {
+        cfg.gridDim = dim3(ctas);
+        cfg.blockDim = dim3(512);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st_;
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        at[1].id = cudaLaunchAttributeClusterDimension;
+        at[1].val.clusterDim.x = ctas;
+        at[1].val.clusterDim.y = 1;
+        at[1].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = ctas > 1 ? 2 : 1;
+    }
+    // whether k_mgs_cycle serves this base grid: 2^3 to 32^3 cells, the
+    // physical-boundary faces those of the boundary module, the shared memory
+    // (and the cluster) available
+    void mgs_init() {
+        int top = 0;
+        while ((2 << top) <= NBc) top++;
+        if (top < 1 || top > 5) return;
+        int want[6];
+        for (int f = 0; f < 6; f++) want[f] = mg.periodic ? 0 : (mg.zbc == 2 && f >= 4 ? 0 : 1);
+        for (int f = 0; f < 6; f++)
+            if (mg.touch[f] != want[f]) return;
+        mgsTop = top;
+        mgsMode = mg.periodic ? kMgPeriodic : (mg.zbc == 1 ? kMgZMirror : (mg.zbc == 2 ? kMgZPeriodic : kMgIsolated));
+        bool ok = true;
+        mgs_with([&](auto kern, int ctas, size_t smem) {
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ok = false;
+            if (ok && ctas > 1) {
+                cudaLaunchConfig_t cfg = {};
+                cudaLaunchAttribute at[2];
+                mgs_config(cfg, at, ctas, smem);
+                cfg.stream = 0;
+                cfg.attrs = at + 1;
+                cfg.numAttrs = 1;
+                int n = 0;
+                if (cudaOccupancyMaxActiveClusters(&n, (const void *)kern, &cfg) != cudaSuccess || n < 1) ok = false;
+            }
+        });
+        if (!ok) {
+            cudaGetLastError();
+            mgsTop = 0;
+        }
     }
     // vmg_fas (vmg.F90:116-243); jrho = IRHS when copy_rhs (second and later calls)
     void vmg_fas(bool copy_rhs) {
