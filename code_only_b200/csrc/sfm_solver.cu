@@ -49,6 +49,7 @@
 #include "sfm_mgs.cuh"
 #include "sfm_fast.cuh"
 #include "sfm_faces.cuh"
+#include "sfm_vmg.cuh"
 #include "sfm_noalloc.cuh"
 #include "sfm_adjoint.cuh"
 #include "sfm_tune.h"
@@ -339,6 +340,10 @@ public:
     CFItem *d_cf = nullptr;
     std::vector<T *> faceBuf[2], cfBuf;
     std::vector<int> facePar;              // buffer holding U[f]'s planes, -1: neither
+    // AMR-level V-cycle by lanes (sfm_vmg.cuh)
+    std::vector<int64_t> cfOff;            // [level] first coarse-fine face of the level
+    uint8_t *d_cropMask = nullptr;
+    T *vmgMargin = nullptr, *vmgAlt = nullptr;
     std::vector<int> leafList;
 
     // fields: inner precision T at every fmg level, FP64 outer fields at level 0
@@ -1114,6 +1119,16 @@ public:
         }
         if (!ok) return;
         facesOk = true;
+        cfOff.assign(H.nlev + 1, 0);
+        std::vector<uint8_t> crop((size_t)H.nb, 0);   // faces of a refined block with a coarse-fine face of a child behind them
+        for (const RefluxItem &r : refl) {
+            cfOff[H.level[r.fine] + 1]++;
+            crop[H.parent[r.fine]] |= (uint8_t)(1 << (r.lr + 2 * r.dir));
+        }
+        for (int L = 0; L < H.nlev; L++) cfOff[L + 1] += cfOff[L];
+        d_cropMask = mem.upload(crop);
+        vmgMargin = mem.alloc<T>(5 * std::max<size_t>(refl.size(), 1));
+        if (sizeof(T) == 4) vmgAlt = mem.alloc<T>((size_t)H.nb * kVB);
         d_fsrc = mem.upload(src);
         d_child = mem.upload(std::vector<int32_t>(H.child.begin(), H.child.end()));
         d_cf = mem.upload(items);
@@ -1919,10 +1934,121 @@ public:
             mgsTop = 0;
         }
     }
+    // ---- the same level operations by lanes (sfm_vmg.cuh) -------------
+    T vmg_h(int L) const { return (T)hlev(H.h0.data(), L, H.FMax); }
+    T vmg_hi(int L) const { return (T)(1.0 / hlev(H.h0.data(), L, H.FMax)); }
+    static unsigned lanes_ctas(int64_t nblk) { return (unsigned)((nblk * 8 + 255) / 256); }
+    int cf_count(int L) const { return L >= 0 && L < H.nlev ? (int)(cfOff[L + 1] - cfOff[L]) : 0; }
+    // coarse-fine ghosts of level L; zeroCoarse: the coarse level is still zero
+    void vmgl_cf(int L, bool zeroCoarse) {
+        const int n = cf_count(L);
+        if (n == 0) return;
+        launch_pdl(k_vmg_cf<T>, (unsigned)((4 * n + 127) / 128), 128, 0, U[H.FMax], (const CFItem *)d_cf + cfOff[L], n,
+                   (const T *)(zeroCoarse ? nullptr : vmgMargin + 5 * cfOff[L]));
+        ++launches;
+    }
+    // snapshot of level L's ghost cells that the coarse-fine faces above it read
+    void vmgl_margin(int L, const T *u) {
+        const int n = cf_count(L + 1);
+        if (n == 0) return;
+        launch_pdl(k_vmg_margin<T>, (unsigned)((n + 127) / 128), 128, 0, u,
+                   (const CFItem *)d_cf + cfOff[L + 1], n, vmgMargin + 5 * cfOff[L + 1]);
+        ++launches;
+    }
+    // nsweep sweeps of level L; snapshot: take the margin before the last launch
+    void vmgl_relax(int L, int nsweep, bool snapshot) {
+        const int F = H.FMax;
+        const bool fused = fused_at(F, 2);
+        const int npass = fused ? 1 : 2, total = nsweep * npass;
+        T *in = U[F], *out = fused ? vmgAlt : U[F];
+        for (int q = 0; q < total; q++) {
+            if (snapshot && q == total - 1) vmgl_margin(L, in);
+            launch_pdl(k_vmg_relax<T>, lanes_ctas(cnt(L)), 256, 0, (const T *)in, out, (const T *)U[F], (const T *)RHS[F],
+                       (const GFace *)d_gface, H.lstart[L], cnt(L), vmg_h(L), vmg_hi(L), q % npass + 1,
+                       fused ? local_sweeps() : 0);
+            ++launches;
+            if (fused) std::swap(in, out);
+        }
+        if (in != U[F]) {   // an odd number of fused launches
+            launch_pdl(k_vmg_copy<T>, lanes_ctas(cnt(L)), 256, 0, U[F], (const T *)in, H.lstart[L], cnt(L));
+            ++launches;
+        }
+    }
+    // down to level v - 1 from level v: relaxation, restriction of U and RHS
+    // with tau (vmg.F90:160-205).  keepGhosts: the same-level ghosts as
+    // vmg_tau leaves them are read later.
+    void vmgl_down(int v, int nsweep, bool keepGhosts) {
+        const int F = H.FMax;
+        vmgl_cf(v, true);
+        vmgl_relax(v, nsweep, false);
+        ghost_fill_level(v, F, U[F], true, -1);   // full shells for the cubic restriction
+        const int64_t wc = wcOff[v] - wcOff[v - 1];
+        launch_pdl(k_vmg_restrict<T>, (unsigned)((8 * wc + 127) / 128), 128, 0, U[F], RHS[F], RES[F],
+                   (const int32_t *)d_withChild + wcOff[v - 1], (int)wc, (const int32_t *)d_child, vmg_hi(v));
+        if (keepGhosts) vmg_ghostcell(v, U[F]);
+        launch_pdl(k_vmg_tau<T>, lanes_ctas(cnt(v - 1)), 256, 0, (const T *)U[F], RUF, RHS[F], (const T *)RES[F],
+                   (const GFace *)d_gface, (const int8_t *)d_skip, (const uint8_t *)d_cropMask, H.lstart[v - 1], cnt(v - 1),
+                   vmg_hi(v - 1));
+        launches += 2;
+    }
+    // the base level
+    void vmgl_base(bool keepGhosts) {
+        const int F = H.FMax;
+        if (P.zero_mean) {
+            if (cnt(0) <= kVmgAveMax) {
+                launch_pdl(k_vmg_zero_average<T>, 1, 1024, 0, RHS[F], cnt(0));
+                ++launches;
+            } else {
+                vmg_zeroAverage(RHS[F]);
+            }
+        }
+        if (useSerialMg) {
+            if (keepGhosts) vmg_ghostcell(0, U[F]);
+            vmgl_margin(0, U[F]);   // vmg_tau's fill is the last before the base solve
+            vmg_slvsml(U[F], RHS[F]);
+        } else if (keepGhosts) {   // ten sweeps, the last with its ghost cells stored
+            vmgl_relax(0, 9, false);
+            vmg_relax(0, U[F], RHS[F]);
+        } else {
+            vmgl_relax(0, 10, true);
+        }
+    }
+    static constexpr int kVmgAveMax = 4096;   // base blocks one CTA averages in the time of the three launches
+    void vmgl_up(int v, int nsweep) {
+        const int F = H.FMax;
+        launch_pdl(k_vmg_correct<T>, lanes_ctas(cnt(v)), 256, 0, U[F], (const T *)RUF, (const GFace *)d_gface,
+                   (const int32_t *)d_parent, (const int8_t *)d_oct, H.lstart[v], cnt(v));
+        ++launches;
+        vmgl_cf(v, false);
+        vmgl_relax(v, nsweep, v < H.nlev - 1);
+    }
     // vmg_fas (vmg.F90:116-243); jrho = IRHS when copy_rhs (second and later calls)
     void vmg_fas(bool copy_rhs) {
         nvtxRangePushA("sfm vmg_fas");
         const int F = H.FMax, nlev = H.nlev;
+        // By lanes: on entry the leaves of U are zero, ghosts included, and
+        // every refined block's U and RHS are restricted from its children
+        // before they are read, so neither is prepared here.  The first
+        // call's ascent keeps the passes: the cubic restriction that follows
+        // it (fmg_interp) reads the ghost shells its sweeps leave.
+        if (facesOk && !serialRelax && nf[F] == 2) {
+            const int nvs = sched(kKnobVmgSweeps, 2);
+            const bool passes = !copy_rhs && nlev > 1;
+            if (!copy_rhs) {   // later calls find the leaves' right-hand side in RHS
+                runB(OpCopy<T, T>{RHS[F], RHO[F], d_leaves, Vf[F]}, nLeaves);
+                boundary_fill0(F, U[F]);
+            }
+            // OpTauFine leaves zero ghosts in RES, which the ascent by passes adds to U's
+            if (passes) runB(OpZero<T>{RES[F], d_all, Vf[F]}, H.nb);
+            for (int v = nlev - 1; v >= 1; v--) vmgl_down(v, nvs, passes);
+            vmgl_base(passes);
+            for (int v = 1; v <= nlev - 1; v++) {
+                if (copy_rhs) vmgl_up(v, nvs);
+                else vmg_up(v, nvs);
+            }
+            nvtxRangePop();
+            return;
+        }
         // the level lists are consecutive ranges of d_all: the per-level
         // copies of vmg_fas are one launch over all blocks
         if (copy_rhs) runB(OpCopy<T, T>{RHO[F], RHS[F], d_all, Vf[F]}, H.nb);
@@ -1944,14 +2070,16 @@ public:
         }
         if (P.zero_mean) vmg_zeroAverage(RHS[F]);
         vmg_slvsml(U[F], RHS[F]);
-        for (int v = 1; v <= nlev - 1; v++) {
-            runB(OpSub<T>{RES[F], U[F], RUF, d_all + H.lstart[v - 1], Vf[F]}, cnt(v - 1));
-            vmg_interp(v, RES[F], RES[F]);
-            runB(OpAdd<T, T>{U[F], RES[F], d_all + H.lstart[v], Vf[F]}, cnt(v));
-            vmg_gridboundary(v, U[F]);
-            for (int q = 0; q < nvs; q++) vmg_relax(v, U[F], RHS[F]);
-        }
+        for (int v = 1; v <= nlev - 1; v++) vmg_up(v, nvs);
         nvtxRangePop();
+    }
+    void vmg_up(int v, int nvs) {   // the correction of level v (vmg.F90:215-240)
+        const int F = H.FMax;
+        runB(OpSub<T>{RES[F], U[F], RUF, d_all + H.lstart[v - 1], Vf[F]}, cnt(v - 1));
+        vmg_interp(v, RES[F], RES[F]);
+        runB(OpAdd<T, T>{U[F], RES[F], d_all + H.lstart[v], Vf[F]}, cnt(v));
+        vmg_gridboundary(v, U[F]);
+        for (int q = 0; q < nvs; q++) vmg_relax(v, U[F], RHS[F]);
     }
 
     // -----------------------------------------------------------------
