@@ -528,4 +528,94 @@ __global__ void __launch_bounds__(256) k_resid_faces(const T *__restrict__ u, co
     for (int t = threadIdx.x; t < nq * VC; t += 256) uc[(int64_t)sbid[t / VC] * VC + t % VC] = (T)0;
 }
 
+// ---------------------------------------------------------------------------
+// the outer FP64 residual (fmg.F90:183, fmg_poisson_resid at level 0) with
+// planes, and the correction's addition that leaves them.  Only on boxes
+// without physical-boundary faces: there the ghosts of psi are not zero.
+// ---------------------------------------------------------------------------
+template <int N>
+__host__ __device__ constexpr int resid_planes_bpc() { return N >= 16 ? 1 : (N == 8 ? 2 : 8); }
+template <class TO, int N>
+__global__ void __launch_bounds__(256) k_resid_planes(TO *__restrict__ res, const double *__restrict__ u,
+                                                      const double *__restrict__ rhs,
+                                                      const int32_t *__restrict__ blocks, int nblk,
+                                                      const double *__restrict__ h0, const int32_t *__restrict__ level,
+                                                      const int32_t *__restrict__ rslot,
+                                                      const double *__restrict__ rbuf, FaceArgs<double> fa) {
+    pdl_enter();
+    constexpr int G = N + 2, NN = N * N, V = G * G * G, CELLS = N * N * N, BPC = resid_planes_bpc<N>();
+    constexpr int LO = 1 + G + G * G, LEN = (N - 1) * LO + 1;   // interior span of a block
+    __shared__ double sh[BPC * V];
+    __shared__ int ssl[BPC][6], sbid[BPC];
+    __shared__ double shi[BPC];
+    __shared__ int8_t hasr[BPC];
+    const int first = blockIdx.x * BPC;
+    const int nq = nblk - first < BPC ? nblk - first : BPC;
+    // the span's cells but its ghost positions (interior ones only), and the
+    // ghost planes: disjoint, so one barrier
+    for (int t = threadIdx.x; t < nq * LEN; t += 256) {
+        const int q = t / LEN, r = t - q * LEN + LO;
+        const int i = r % G, j = (r / G) % G;
+        const double v = u[(int64_t)blocks[first + q] * V + r];
+        if (i >= 1 && i <= N && j >= 1 && j <= N) sh[q * V + r] = v;
+    }
+    for (int t = threadIdx.x; t < nq * 6 * NN; t += 256) {
+        const int q = t / (6 * NN), r = t - q * (6 * NN), fc = r / NN, e = r - fc * NN;
+        const int v = fa.src[6 * (int64_t)blocks[first + q] + fc];
+        int i, j, k;
+        put3(fc >> 1, (fc & 1) ? N : -1, e % N, e / N, i, j, k);
+        sh[q * V + cidx(G, i, j, k)] =
+            v >= 0 ? fa.in[(int64_t)v * NN + e] : (v == kFaceZero ? 0.0 : fa.cf[(int64_t)(-2 - v) * NN + e]);
+    }
+    if ((int)threadIdx.x < nq) {
+        const int q = threadIdx.x, b = blocks[first + q];
+        int any = 0;
+        for (int fc = 0; fc < 6; fc++) {
+            const int v = rslot[6 * (int64_t)b + fc];
+            ssl[q][fc] = v;
+            any |= v >= 0;
+        }
+        sbid[q] = b;
+        hasr[q] = (int8_t)any;
+        shi[q] = 1.0 / hlev(h0, level[b], 0);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < nq * CELLS; t += 256) {
+        const int q = t / CELLS, r = t - q * CELLS;
+        const int i = r % N, j = (r / N) % N, k = r / NN;
+        const double hi = shi[q];
+        const TileFlux<double, N> F{sh + q * V, hi, hasr[q] ? ssl[q] : nullptr, rbuf};
+        const int64_t c = (int64_t)sbid[q] * V + cidx(G, i, j, k);
+        res[c] = (TO)(rhs[c] - F.div(i, j, k) * hi);
+    }
+}
+template <class T, int N>
+__global__ void __launch_bounds__(256) k_add_planes(double *__restrict__ a, const T *__restrict__ d,
+                                                    const int32_t *__restrict__ blocks, int nblk,
+                                                    double *__restrict__ planes) {
+    pdl_enter();
+    constexpr int G = N + 2, CELLS = N * N * N, PER = CELLS / 256 > 0 ? CELLS / 256 : 1;
+    constexpr int BPC = CELLS >= 256 ? 1 : 256 / CELLS;   // blocks per step of a CTA
+    constexpr int64_t V = (int64_t)G * G * G;
+    for (int b0 = blockIdx.x * BPC; b0 < nblk; b0 += gridDim.x * BPC) {
+        const int q = b0 + (int)threadIdx.x / CELLS;
+        if (q >= nblk) continue;
+        const int64_t b = blocks[q];
+        double v[PER];
+#pragma unroll
+        for (int x = 0; x < PER; x++) {
+            const int r = (int)threadIdx.x % CELLS + 256 * x;
+            const int64_t c = b * V + cidx(G, r % N, (r / N) % N, r / (N * N));
+            v[x] = a[c] + (double)d[c];
+        }
+#pragma unroll
+        for (int x = 0; x < PER; x++) {
+            const int r = (int)threadIdx.x % CELLS + 256 * x;
+            const int i = r % N, j = (r / N) % N, k = r / (N * N);
+            a[b * V + cidx(G, i, j, k)] = v[x];
+            faces_put<double, N>(planes, b, i, j, k, v[x]);
+        }
+    }
+}
+
 }  // namespace sfm

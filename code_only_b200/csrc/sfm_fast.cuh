@@ -493,7 +493,9 @@ __device__ __noinline__ T ghost_cf_face(const T *u, const int8_t *oct, int X, in
 // The remaining CTAs take the general items.
 constexpr int kGhostWarps = 8;   // blocks per sweep CTA (one per warp)
 template <int N>
-__host__ __device__ constexpr int ghost_sweep_ctas(int nblk) { return (nblk + kGhostWarps - 1) / kGhostWarps; }
+__host__ __device__ constexpr int ghost_sweep_ctas(int nblk) {
+    return (nblk + kGhostWarps - 1) / kGhostWarps;
+}
 template <int N>
 __host__ __device__ constexpr int ghost_general_ctas(int items) {
     return (int)(((int64_t)items * N + 255) / 256);   // N cells per item (corners use the first)
@@ -1345,42 +1347,82 @@ __global__ void __launch_bounds__(256) k_converge_tiled(T *__restrict__ u, const
 // ---------------------------------------------------------------------------
 constexpr int kSumChunk = 1024;
 
-// leaf mean: sum_b psum_b dv_b / sum_b n^3 dv_b over the listed blocks
+// leaf mean: sum_b psum_b dv_b / vol over the listed blocks (vol: the ordered
+// sum of n^3 dv_b, formed once on the host).  Bound by the chain of dependent
+// adds, 8 cycles each.
 __global__ void __launch_bounds__(1024) k_mean_combine_w(const double *__restrict__ psum,
                                                          const int32_t *__restrict__ blocks, int nblk,
                                                          const int32_t *__restrict__ level,
-                                                         const double *__restrict__ h0, int n, double *out) {
+                                                         const double *__restrict__ h0, double vol, double *out) {
     pdl_enter();
-    __shared__ double tm[2][kSumChunk], tv[2][kSumChunk];
+    constexpr int U = 16;
+    __shared__ __align__(16) double tm[2][kSumChunk];
     const int tid = threadIdx.x;
-    const double ncell = (double)(n * n * n);
     const int nch = (nblk + kSumChunk - 1) / kSumChunk;
-    auto stage = [&](int c) {
+    auto stage = [&](int c) {   // past the end: +0, which changes no running sum that started at +0
         for (int t = tid - 32; t < kSumChunk; t += (int)blockDim.x - 32) {
             const int b = c * kSumChunk + t;
-            if (b >= nblk) break;
-            const double hd = h0[level[blocks[b]]];
-            const double dv = hd * hd * hd;
-            tm[c & 1][t] = psum[b] * dv;
-            tv[c & 1][t] = ncell * dv;
+            double v = 0.0;
+            if (b < nblk) {
+                const double hd = h0[level[blocks[b]]];
+                const double dv = hd * hd * hd;
+                v = psum[b] * dv;
+            }
+            tm[c & 1][t] = v;
         }
     };
-    double mass = 0.0, vol = 0.0;
+    double mass = 0.0;
     if (tid >= 32 && nch > 0) stage(0);
     __syncthreads();
     for (int c = 0; c < nch; c++) {
         if (tid >= 32) {
             if (c + 1 < nch) stage(c + 1);
         } else if (tid == 0) {
+            const double2 *q = reinterpret_cast<const double2 *>(tm[c & 1]);
             const int cnt = nblk - c * kSumChunk < kSumChunk ? nblk - c * kSumChunk : kSumChunk;
-            for (int q = 0; q < cnt; q++) {
-                mass = mass + tm[c & 1][q];
-                vol = vol + tv[c & 1][q];
+            for (int e = 0; e < cnt; e += U) {
+                double2 v[U / 2];
+#pragma unroll
+                for (int x = 0; x < U / 2; x++) v[x] = q[e / 2 + x];
+#pragma unroll
+                for (int x = 0; x < U / 2; x++) {
+                    mass = mass + v[x].x;
+                    mass = mass + v[x].y;
+                }
             }
         }
         __syncthreads();
     }
     if (tid == 0) *out = mass / vol;
+}
+
+// Sums over the interiors of the listed blocks, each in Fortran SUM order (i
+// fastest): a lane per block adds from shared memory, one plane of 32 blocks
+// at a time staged by coalesced loads (a thread per block straight from
+// global memory touches 32 blocks' rows per load).
+template <int N>
+__global__ void __launch_bounds__(128) k_block_sums(const double *__restrict__ a, const int32_t *__restrict__ blocks,
+                                                    int nblk, double *__restrict__ out) {
+    pdl_enter();
+    constexpr int G = N + 2, ROWS = N >= 16 ? 4 : N, P = ROWS * N + 1;   // values of a staged piece, padded
+    constexpr int64_t V = (int64_t)G * G * G;
+    __shared__ double sh[32 * P];
+    __shared__ int sb[32];
+    const int first = blockIdx.x * 32, nq = nblk - first < 32 ? nblk - first : 32;
+    if ((int)threadIdx.x < nq) sb[threadIdx.x] = blocks[first + threadIdx.x];
+    double s = 0.0;
+    for (int k = 0; k < N; k++)
+        for (int j0 = 0; j0 < N; j0 += ROWS) {
+            __syncthreads();
+            for (int t = threadIdx.x; t < nq * ROWS * N; t += 128) {
+                const int q = t / (ROWS * N), r = t - q * (ROWS * N);
+                sh[q * P + r] = a[sb[q] * V + cidx(G, r % N, j0 + r / N, k)];
+            }
+            __syncthreads();
+            if ((int)threadIdx.x < nq)
+                for (int r = 0; r < ROWS * N; r++) s = s + sh[threadIdx.x * P + r];
+        }
+    if ((int)threadIdx.x < nq) out[first + threadIdx.x] = s;
 }
 
 // base-level average: sum_b psum_b / (n^3 nblk)

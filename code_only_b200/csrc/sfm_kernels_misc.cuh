@@ -25,6 +25,33 @@ struct OpPhysvar {
     }
 };
 
+// The same straight into the outer solve's fields: PSI := psi and SRC :=
+// rho * 4 pi G on leaves (refined blocks get theirs by restriction); every
+// block's input is checked.  A CTA per block, 32-bit index arithmetic.
+__global__ void __launch_bounds__(256) k_physvar(double *__restrict__ PSI, double *__restrict__ SRC,
+                                                 const double *__restrict__ rho, const double *__restrict__ psi,
+                                                 const int8_t *__restrict__ skip, int nb, int n, int g, double fourpiG,
+                                                 int *bad) {
+    pdl_enter();
+    const int G = n + 2, V = G * G * G, Gi = n + 2 * g;
+    const int64_t Vi = (int64_t)Gi * Gi * Gi;
+    bool odd = false;
+    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+        const bool leaf = !skip[b];
+        for (int e = threadIdx.x; e < V; e += 256) {
+            const int r = e / G, i = e - r * G, k = r / G, j = r - k * G;
+            const int64_t s = b * Vi + ((k + g - 1) * Gi + (j + g - 1)) * Gi + (i + g - 1);
+            const double rv = rho[s], pv = psi ? psi[s] : 0.0;
+            odd = odd || !isfinite(rv) || !isfinite(pv);
+            if (leaf) {
+                PSI[(int64_t)b * V + e] = pv;
+                SRC[(int64_t)b * V + e] = rv * fourpiG;
+            }
+        }
+    }
+    if (odd) *bad = 1;
+}
+
 // per-block interior sum, sequential in (i fastest) order as Fortran SUM
 template <class T>
 struct OpBlockSum {
@@ -39,35 +66,24 @@ struct OpBlockSum {
     }
 };
 
-// leaf-volume mean of RHO (fmg_data_if.F90:59-77): mass and volume summed
-// block after block in level order, then rho_ave -> *out
-__global__ void k_mean_combine(const double *psum, const int32_t *blocks, int nblk, const int32_t *level,
-                               const double *h0, int n, double *out) {
-    pdl_enter();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double mass = 0.0, vol = 0.0;
-    for (int q = 0; q < nblk; q++) {
-        double hd = h0[level[blocks[q]]];
-        double dv = hd * hd * hd;
-        mass = mass + psum[q] * dv;
-        vol = vol + (double)(n * n * n) * dv;
-    }
-    *out = mass / vol;
-}
-
-// vmg_zeroAverage (vmg.F90:900-916) via fmg_ave (fmg_data.F90:730-769)
-__global__ void k_ave_combine(const double *psum, int nblk, int n, double *out) {
-    pdl_enter();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double ave = 0.0;
-    for (int q = 0; q < nblk; q++) ave = ave + psum[q];
-    *out = nblk == 0 ? 0.0 : ave / (double)(n * n * n * nblk);
-}
-
 template <class T>
 struct OpSubScalarAll {      // a := a - *s over whole arrays
     T *a; const double *s;
     __device__ void operator()(int64_t idx) const { a[idx] = a[idx] - (T)(*s); }
+};
+struct OpSubScalarBlocks {   // a := a - *s over whole listed blocks
+    double *a; const double *s; const int32_t *blocks; int64_t V;
+    static constexpr int VW = 2;
+    __device__ void cell(int64_t c) const { a[c] = a[c] - *s; }
+    template <int W>
+    __device__ void cells(int64_t c) const {
+        double x[W];
+        vec_load<double, W>(a + c, x);
+#pragma unroll
+        for (int i = 0; i < W; i++) x[i] = x[i] - *s;
+        vec_store<double, W>(a + c, x);
+    }
+    bool aligned() const { return aligned16(a); }
 };
 template <class T>
 struct OpSubScalarInterior { // a := a - *s on the interior of consecutive blocks

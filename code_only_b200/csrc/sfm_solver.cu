@@ -340,11 +340,17 @@ public:
     CFItem *d_cf = nullptr;
     std::vector<T *> faceBuf[2], cfBuf;
     std::vector<int> facePar;              // buffer holding U[f]'s planes, -1: neither
+    // the outer residual's (boxes without physical-boundary faces): planes of PSI0
+    double *outerPlanes = nullptr, *outerCf = nullptr;
+    // whole arrays as the reference leaves them, unread ghost cells and
+    // refined blocks included (the debug entry's stage dumps compare them)
+    bool wholeArrays = false;
     // AMR-level V-cycle by lanes (sfm_vmg.cuh)
     std::vector<int64_t> cfOff;            // [level] first coarse-fine face of the level
     uint8_t *d_cropMask = nullptr;
     T *vmgMargin = nullptr, *vmgAlt = nullptr;
     std::vector<int> leafList;
+    double leafVol = 0.0;
 
     // fields: inner precision T at every fmg level, FP64 outer fields at level 0
     std::vector<T *> U, RES, RHS, RHO;
@@ -473,11 +479,59 @@ public:
     void outer_iteration_body() {
         nvtxRangePushA("sfm outer iteration");
         profNext = 0;
-        resid<double, double, T>(0, RHO[0], PSI0, SRC0, false);
-        fmg_lin();
-        add(0, PSI0, U[0]);
+        if (outerPlanes && !wholeArrays) {
+            outer_resid_planes();
+            fmg_lin();
+            outer_add_planes();
+        } else {
+            resid<double, double, T>(0, RHO[0], PSI0, SRC0, false);
+            fmg_lin();
+            add(0, PSI0, U[0]);
+        }
         profPairs = profNext;
         nvtxRangePop();
+    }
+    template <class F>
+    void with_outer_edge(F &&go) {
+        switch (H.NI) {
+            case 4: go(std::integral_constant<int, 4>{}); break;
+            case 8: go(std::integral_constant<int, 8>{}); break;
+            default: go(std::integral_constant<int, 16>{}); break;
+        }
+    }
+    void outer_planes_of() {   // the planes of PSI0 as it stands
+        with_outer_edge([&](auto e) {
+            constexpr int N = decltype(e)::value;
+            launch_pdl(k_faces_of<double, N>,
+                       (unsigned)std::min<int64_t>(((int64_t)nLeaves * 6 * N * N + 255) / 256, (int64_t)nSM * 16), 256, 0,
+                       (const double *)PSI0, outerPlanes, (const int32_t *)d_leaves, nLeaves);
+            ++launches;
+        });
+    }
+    void outer_resid_planes() {
+        with_outer_edge([&](auto e) {
+            constexpr int N = decltype(e)::value;
+            if (nReflux > 0) {
+                launch_pdl(k_cf_reflux<double, N>, (unsigned)(((int64_t)nReflux * (N / 2) * (N / 2) + 127) / 128), 128, 0,
+                           (const double *)PSI0, (const double *)outerPlanes, outerCf, rbuf[0], (const CFItem *)d_cf,
+                           nReflux, (const int32_t *)d_child, (const double *)d_h0, (const int32_t *)d_level, 0);
+                ++launches;
+            }
+            const FaceArgs<double> fa{outerPlanes, nullptr, outerCf, nullptr, d_fsrc, 0};
+            launch_pdl(k_resid_planes<T, N>, (unsigned)((nLeaves + resid_planes_bpc<N>() - 1) / resid_planes_bpc<N>()), 256,
+                       0, RHO[0], (const double *)PSI0, (const double *)SRC0, (const int32_t *)d_leaves, nLeaves,
+                       (const double *)d_h0, (const int32_t *)d_level, (const int32_t *)d_rslot, (const double *)rbuf[0],
+                       fa);
+            ++launches;
+        });
+    }
+    void outer_add_planes() {
+        with_outer_edge([&](auto e) {
+            constexpr int N = decltype(e)::value;
+            launch_pdl(k_add_planes<T, N>, (unsigned)std::min(nLeaves, nSM * 16), 256, 0, PSI0, (const T *)U[0],
+                       (const int32_t *)d_leaves, nLeaves, outerPlanes);
+            ++launches;
+        });
     }
     void outer_iteration() {
         if (graphsOff) { outer_iteration_body(); return; }
@@ -720,6 +774,9 @@ public:
             }
             tune.set(kKnobBaseCtas, (int)sizeof(T), NBc, -1, -1, pick.nct);
             tune.set(kKnobBaseWide, (int)sizeof(T), NBc, -1, -1, pick.wide);
+        } else if (useSerialMg) {   // k_mgs_cycle: one shape per base grid, recorded as it is
+            tune.set(kKnobBaseCtas, (int)sizeof(T), NBc, -1, -1, mgsTop >= 5 ? 8 : 1);
+            tune.set(kKnobBaseWide, (int)sizeof(T), NBc, -1, -1, 16);
         }
         FmgLevel_fill0 = Undef;
         if (iterExec) {   // the graph holds the old launch shapes
@@ -992,6 +1049,16 @@ public:
             if (nn && cfBuf.back() && cudaMemset(cfBuf.back() + (size_t)nReflux * nn, 0, nn * sizeof(T)) != cudaSuccess)
                 mem.err = cudaErrorUnknown;
             facePar.push_back(-1);
+        }
+        if (facesOk && tfL.empty() && (H.NI == 4 || H.NI == 8 || H.NI == 16)) {
+            const size_t nn = (size_t)H.NI * H.NI;
+            outerPlanes = mem.alloc<double>((size_t)nb * 6 * nn);
+            outerCf = mem.alloc<double>((size_t)std::max(nReflux, 1) * nn);
+        }
+        for (int b : leafList) {   // the ordered volume sum of the leaf mean (fmg_data_if.F90:59-77)
+            const double hd = H.h0[H.level[b]];
+            const double dv = hd * hd * hd;
+            leafVol = leafVol + (double)(H.NI * H.NI * H.NI) * dv;
         }
         RUF = fieldT(FMax);
         SRC0 = fieldD(0); PSI0 = fieldD(0); PHI0 = fieldD(0); RES0d = fieldD(0);
@@ -1708,9 +1775,9 @@ public:
 
     // the descent step of fmg_lin: residual of level v restricted to the next
     // level's right-hand side, that level's correction zeroed
-    void resid_rstrct_fill0(int v) {
+    void resid_rstrct_fill0(int v, T *rhs) {
         if (!faces_at(v)) {
-            resid(v, RES[v], U[v], RHS[v], true);
+            resid(v, RES[v], U[v], rhs, true);
             fmg_rstrct(v + 1, RHS[v + 1], RES[v]);
             fill0(v + 1, U[v + 1]);
         } else {
@@ -1719,7 +1786,7 @@ public:
                 constexpr int N = decltype(edge)::value;
                 if constexpr (bulk_ok<N>()) {
                     launch_pdl(k_resid_faces<T, N>, (unsigned)((nLeaves + resid_faces_bpc<N>() - 1) / resid_faces_bpc<N>()),
-                               256, 0, (const T *)U[v], (const T *)RHS[v], RHS[v + 1], U[v + 1],
+                               256, 0, (const T *)U[v], (const T *)rhs, RHS[v + 1], U[v + 1],
                                (const int32_t *)d_leaves, nLeaves, (const double *)d_h0, (const int32_t *)d_level,
                                (const int32_t *)d_rslot, (const double *)rbuf[v], face_args(v, false), v);
                     ++launches;
@@ -1739,12 +1806,14 @@ public:
         vmg_fas(false);
         for (int f = FMax - 1; f >= 0; f--) {
             fmg_interp(f, U[f], U[f + 1], true);
-            copy(f, RHS[f], RHO[f], false);
+            // the reference copies RHO to RHS on level f (fmg.F90:290); the
+            // sweeps and residuals there read RHO itself
+            auto rhs = [&](int v) { return v == f ? RHO[v] : RHS[v]; };
             const int ncycle = sched(kKnobFmgCycles, 2), nsweep = sched(kKnobFmgSweeps, 2);
             for (int jc = 1; jc <= ncycle; jc++) {
                 for (int v = f; v <= FMax - 1; v++) {
-                    for (int q = 0; q < nsweep; q++) relax(v, U[v], RHS[v], true, 4, false);
-                    resid_rstrct_fill0(v);
+                    for (int q = 0; q < nsweep; q++) relax(v, U[v], rhs(v), true, 4, false);
+                    resid_rstrct_fill0(v, rhs(v));
                 }
                 vmg_fas(true);
                 for (int v = FMax - 1; v >= f; v--) {
@@ -1756,16 +1825,15 @@ public:
                     }
                     for (int q = 0; q < nsweep; q++) {
                         // the level's last sweep: the cubic restriction of the
-                        // next fmg level (level 0: the caller) reads the ghost
-                        // layer it leaves, and level 0's maximum is the one
-                        // the stopping rule takes
+                        // next fmg level reads the ghost layer it leaves, and
+                        // level 0's maximum is the one the stopping rule takes
                         const bool last = jc == ncycle && v == f && q == nsweep - 1;
-                        relax(v, U[v], RHS[v], true, last && v == 0 ? 0 : 4, last);
+                        relax(v, U[v], rhs(v), true, last && v == 0 ? 0 : 4, last && (v > 0 || wholeArrays));
                     }
                 }
             }
         }
-        converge_c2p(0, U[0]);
+        if (wholeArrays) converge_c2p(0, U[0]);   // only the leaves' correction is used
         nvtxRangePop();
     }
 
@@ -1854,7 +1922,9 @@ public:
         }
         int64_t N3 = (int64_t)NBc * NBc * NBc;
         run(OpMgGather<T>{mg.SRC, mg.PSI, rhs, u, d_baseIdx, H.ngb[0], H.ngb[1], nf[F], Gf[F], NBc, Vf[F]}, N3);
-        mg_launch(tune.get(kKnobBaseCtas, (int)sizeof(T), NBc, -1, -1, 1),
+        // default: the largest cluster from 32 cells per edge on (64^3 base
+        // grid: 136 ms a solve on one CTA, 45 ms on 16)
+        mg_launch(tune.get(kKnobBaseCtas, (int)sizeof(T), NBc, -1, -1, NBc >= 32 && mg_fits(16, 16) ? 16 : 1),
                   tune.get(kKnobBaseWide, (int)sizeof(T), NBc, -1, -1, 16));
         run(OpMgScatter<T>{u, mg.PSI, d_baseIdx, H.ngb[0], H.ngb[1], nf[F], Gf[F], NBc, Vf[F]}, N3);
     }
@@ -2174,20 +2244,43 @@ public:
         for (auto &z : zeroList) cudaMemsetAsync(z.first, 0, z.second, st_);
         cudaMemsetAsync(d_bad, 0, sizeof(int), st_);
         FmgLevel_fill0 = Undef;
+        if (wholeArrays != (stop_stage != 0)) {   // the iteration's graph was captured for the other
+            wholeArrays = stop_stage != 0;
+            if (iterExec) {
+                cudaGraphExecDestroy(iterExec);
+                iterExec = nullptr;
+            }
+        }
         // fmg_make_physvar
-        run(OpPhysvar<double>{PHI0, RES0d, rho, psi, H.NI, Gf[0], gw, Vf[0], P.four_pi_G, d_bad}, (int64_t)nb * Vf[0]);
-        if (P.zero_mean) {
-            run(OpBlockSum<double>{RES0d, d_leaves, d_psum, H.NI, Gf[0], Vf[0]}, (int64_t)nLeaves);
-            launch_pdl(k_mean_combine_w, 1, 1024, 0, d_psum, d_leaves, nLeaves, d_level, d_h0, H.NI, d_scal);
+        if (wholeArrays)
+            run(OpPhysvar<double>{PHI0, RES0d, rho, psi, H.NI, Gf[0], gw, Vf[0], P.four_pi_G, d_bad}, (int64_t)nb * Vf[0]);
+        else {
+            launch_pdl(k_physvar, (unsigned)std::min(nb, nSM * 16), 256, 0, PSI0, SRC0, rho, (const double *)psi,
+                       (const int8_t *)d_skip, nb, H.NI, gw, P.four_pi_G, d_bad);
             ++launches;
-            run(OpSubScalarAll<double>{RES0d, d_scal}, (int64_t)nb * Vf[0]);
+        }
+        if (P.zero_mean) {
+            const double *R = wholeArrays ? RES0d : SRC0;
+            SFM_WITH_N(H.NI,
+                       (launch_pdl(k_block_sums<N>, (unsigned)((nLeaves + 31) / 32), 128, 0, R, (const int32_t *)d_leaves,
+                                   nLeaves, d_psum),
+                        ++launches),
+                       run(OpBlockSum<double>{R, d_leaves, d_psum, H.NI, Gf[0], Vf[0]}, (int64_t)nLeaves))
+            launch_pdl(k_mean_combine_w, 1, 1024, 0, d_psum, d_leaves, nLeaves, d_level, d_h0, leafVol, d_scal);
+            ++launches;
+            if (wholeArrays) run(OpSubScalarAll<double>{RES0d, d_scal}, (int64_t)nb * Vf[0]);
+            else runB(OpSubScalarBlocks{SRC0, d_scal, d_leaves, Vf[0]}, nLeaves);
         } else {
             cudaMemsetAsync(d_scal, 0, sizeof(double), st_);
         }
-        copy(0, RHO[0], RES0d, true);   // IRHO(f0) as the reference holds it
-        copy(0, U[0], PHI0, true);      // IU(f0)
-        copy(0, PSI0, PHI0, false);     // fmg_copy(IPSI, IU)
-        copy(0, SRC0, RES0d, false);    // fmg_copy(ISRC, IRHO)
+        // the reference's copies of RHO and U (fmg_copy, fmg.F90:150-160): what
+        // the solve reads of them is rewritten before
+        if (wholeArrays) {
+            copy(0, RHO[0], RES0d, true);   // IRHO(f0) as the reference holds it
+            copy(0, U[0], PHI0, true);      // IU(f0)
+            copy(0, PSI0, PHI0, false);     // fmg_copy(IPSI, IU)
+            copy(0, SRC0, RES0d, false);    // fmg_copy(ISRC, IRHO)
+        }
         converge_c2p(0, SRC0);
         converge_c2p(0, PSI0);
         boundary_physical_grid();
@@ -2207,6 +2300,7 @@ public:
         if (std::fabs(resh2max) <= std::numeric_limits<double>::min()) nmax = 0;
         bool conv = true, reached = (nmax == 0);
         int iters = 0;
+        if (outerPlanes && !wholeArrays && nmax > 0) outer_planes_of();
         for (int it = 1; it <= nmax; it++) {
             if (stop_stage == 2 || stop_stage == 3) {
                 resid<double, double, T>(0, RHO[0], PSI0, SRC0, false);
