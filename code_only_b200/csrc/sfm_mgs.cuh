@@ -67,6 +67,60 @@ struct Mgs {
         const Tables *t;
         int rank;              // CTA in the cluster
     };
+    static __device__ __forceinline__ void fill_tables(Tables &t, double hbase) {
+        for (int e = threadIdx.x; e < (2 << TOP); e += blockDim.x) {   // entry n + i of level n >= 4
+            int n = 4;
+            while (2 * n <= e) n *= 2;
+            if (e >= 4) cubic_weights(e - n, -1, n / 2, t.c[e], t.w[e]);
+        }
+        if ((int)threadIdx.x <= TOP) {
+            const double hh = hbase * (double)(1 << (TOP - (int)threadIdx.x));
+            t.h2[threadIdx.x] = hh * hh;
+            t.h2i[threadIdx.x] = 1.0 / (hh * hh);
+        }
+    }
+    static __device__ __forceinline__ void meet() {   // everyone who holds a part of the finest level
+        if (C > 1) mg_cluster_sync();
+        else __syncthreads();
+    }
+    // maximum over the cluster; red (32 values) and slot in shared memory
+    static __device__ __forceinline__ double vmax(double v, double *red, double *slot) {
+        v = mg_block_max(v, red);
+        if (C > 1) {
+            if (threadIdx.x == 0) *slot = v;
+            mg_cluster_sync();
+            for (int q = 0; q < C; q++) {
+                const double t = *mg_map_rank(slot, q);
+                v = t > v ? t : v;
+            }
+            mg_cluster_sync();
+        }
+        return v;
+    }
+    // residual of PSI into the finest RHO; this thread's maximum
+    static __device__ __forceinline__ double defect(const Ctx &x) {
+        constexpr int N = 1 << TOP;
+        double v = 0.0;
+        for (int c = threadIdx.x; c < vol(TOP); c += blockDim.x) {
+            const double r = resid<TOP>(x, PSI, SRC, c & (N - 1), (c >> TOP) & (N - 1), c >> (2 * TOP));
+            sm()[RHO(TOP) + c] = r;
+            const double q = fabs(r);
+            v = q > v ? q : v;
+        }
+        return v;
+    }
+    // mg_lin (mg.F90:106-218) for the residual in RHO, its correction added
+    // to PSI; this thread's max |resh2| of the last sweep
+    static __device__ __forceinline__ double correct(const Ctx &x) {
+        double rm = 0.0;
+        if (TOP >= 3 || threadIdx.x < 32) {   // base grids of at most 4^3 cells: one warp
+            rstrct_rho<TOP>(x);
+            rm = fmg<TOP>(x);
+        }
+        if (TOP < 3) __syncthreads();
+        for (int c = threadIdx.x; c < vol(TOP); c += blockDim.x) sm()[PSI + c] = sm()[PSI + c] + sm()[U(TOP) + c];
+        return rm;
+    }
     // this CTA's arrays (the symbol itself, so that accesses are shared loads and not generic ones)
     static __device__ __forceinline__ double *sm() {
         extern __shared__ double mgs_smem[];
@@ -330,16 +384,7 @@ __global__ void __launch_bounds__(512, 1) k_mgs_cycle(T *__restrict__ ub, const 
     constexpr int N = 1 << TOP, P = M::planes(TOP), VOL = M::vol(TOP);
     const int tid = threadIdx.x, rank = C > 1 ? mg_cluster_rank() : 0;
     const typename M::Ctx x{&tab, rank};
-    for (int e = tid; e < (2 << TOP); e += 512) {   // entry n + i of level n >= 4
-        int n = 4;
-        while (2 * n <= e) n *= 2;
-        if (e >= 4) cubic_weights(e - n, -1, n / 2, tab.c[e], tab.w[e]);
-    }
-    if (tid <= TOP) {
-        const double hh = a.hbase * (double)(1 << (TOP - tid));
-        tab.h2[tid] = hh * hh;
-        tab.h2i[tid] = 1.0 / (hh * hh);
-    }
+    M::fill_tables(tab, a.hbase);
     auto cell = [&](int c) -> int64_t {   // the block cell of this CTA's base cell c
         const int I = c & (N - 1), J = (c >> TOP) & (N - 1), K = (c >> (2 * TOP)) + rank * P;
         const int ib = I / a.n, jb = J / a.n, kb = K / a.n;
@@ -350,46 +395,16 @@ __global__ void __launch_bounds__(512, 1) k_mgs_cycle(T *__restrict__ ub, const 
         mgs_smem[M::SRC + c] = (double)rhsb[b];
         mgs_smem[M::PSI + c] = (double)ub[b];
     }
-    auto meet = [&]() {
-        if (C > 1) mg_cluster_sync();
-        else __syncthreads();
-    };
-    auto vmax = [&](double v) -> double {   // over the cluster
-        v = mg_block_max(v, red);
-        if (C > 1) {
-            if (tid == 0) slot = v;
-            mg_cluster_sync();
-            for (int q = 0; q < C; q++) {
-                const double t = *mg_map_rank(&slot, q);
-                v = t > v ? t : v;
-            }
-            mg_cluster_sync();
-        }
-        return v;
-    };
-    meet();
+    M::meet();
     const double errmax = (double)1.e-2f;   // default-real literal (mg.F90:50)
     double rhomax = 0.0;
     for (int it = 1; it <= a.nmax; it++) {
-        double v = 0.0;
-        for (int c = tid; c < VOL; c += 512) {
-            const double r = M::template resid<TOP>(x, M::PSI, M::SRC, c & (N - 1), (c >> TOP) & (N - 1), c >> (2 * TOP));
-            mgs_smem[M::RHO(TOP) + c] = r;
-            const double q = fabs(r);
-            v = q > v ? q : v;
-        }
-        meet();
-        if (it == 1) rhomax = vmax(v);
-        double rm = 0.0;
-        if (TOP >= 3 || tid < 32) {   // base grids of at most 4^3 cells: one warp
-            M::template rstrct_rho<TOP>(x);
-            rm = M::template fmg<TOP>(x);
-        }
-        if (TOP < 3) __syncthreads();
+        const double v = M::defect(x);
+        M::meet();
+        if (it == 1) rhomax = M::vmax(v, red, &slot);
+        const double rm = M::correct(x);
         const double hh = a.hbase;
-        const double res = vmax(rm) / (hh * hh);
-        for (int c = tid; c < VOL; c += 512) mgs_smem[M::PSI + c] = mgs_smem[M::PSI + c] + mgs_smem[M::U(TOP) + c];
-        meet();
+        const double res = M::vmax(rm, red, &slot) / (hh * hh);   // PSI is complete after it
         if (res / rhomax < errmax) break;
     }
     for (int c = tid; c < VOL; c += 512) ub[cell(c)] = (T)mgs_smem[M::PSI + c];

@@ -5,149 +5,130 @@
 // solve: code running inside a fixed memory pool or an arena handed out at
 // start-up, a real-time step whose allocator calls would synchronise the
 // device, or a host library that has promised its user a fixed device
-// footprint.  For them this entry point runs the base-grid multigrid of
-// sfm_mg.cuh (mg_lin as repeated defect corrections, mg.F90:42-94) on the
-// caller's device buffers, with every working array in one file-scope
-// __device__ array of fixed size.  Nothing is allocated: no cudaMalloc, no
-// cudaFree, no allocating library call.  The only set-up is the lookup of
-// that array's device address, once per device (cudaGetSymbolAddress).
+// footprint.  For them this entry point runs the base-grid multigrid
+// (mg_lin as repeated defect corrections, mg.F90:42-94) on the caller's
+// device buffers, with every working array in shared memory (sfm_mgs.cuh):
+// one CTA up to 16^3 cells, a cluster of 8 CTAs for 32^3.  Nothing is
+// allocated: no cudaMalloc, no cudaFree, no allocating library call.  The
+// only set-up is, once per device, the lookup of the two result words'
+// address and the kernels' shared-memory opt-in.
 //
 // Limits and contract:
 //   - n (cells per edge) is a power of two, 2 <= n <= SFM_NOALLOC_MAX_N (32);
-//     the scratch holds the level arrays for n = 32, about 2 MiB;
-//   - the kernel clears every scratch array it reads before its first read,
-//     so the scratch needs no zeroing by the caller and no state carries
-//     over from one call to the next;
-//   - there is one scratch array per device and loaded library: two calls on
-//     the same device whose executions overlap (different streams without an
-//     ordering between them, or different host threads) race on it and give
-//     wrong results.  Order such calls on one stream or with events;
-//   - the first call on each device does the set-up lookup; make that first
-//     call before any stream capture on that device.
+//   - no state carries over from one call to the next;
+//   - the two result words (residual, cycle count) are one pair per device
+//     and loaded library: of two calls on the same device whose executions
+//     overlap, the host outputs of either may be the other's.  Order calls
+//     that ask for host outputs on one stream or with events;
+//   - the first call on each device does the set-up; make that first call
+//     before any stream capture on that device.
+//
+// Bound by the serial chain of colour sweeps and transfers (about 400
+// dependent steps a cycle).  A call at n = 32 and rel_tol 1e-10: 2.83 ms with
+// the level arrays in global memory on one CTA of 1024 threads, 0.58 ms here
+// (2.2 ms of the first figure hid the host's 2.5 ms device query, which is
+// gone too; the kernel alone went from 2.1 to 0.55 ms).
 #pragma once
-#include "sfm_mg.cuh"
+#include "sfm_mgs.cuh"
 
 namespace sfm {
 
 constexpr int NOALLOC_MAX_N = 32;
+static __device__ double g_noalloc_out[2];   // relative residual and cycle count
 
-// doubles of the U/RES/RHS/RHO arrays of every level of an n^3 base grid,
-// plus SRC and PSI on level 0
-__host__ __device__ constexpr size_t noalloc_level_doubles(int n) {
-    size_t tot = 0;
-    for (int m = 0; (n >> m) >= 1; m++) {
-        const size_t G = (size_t)(n >> m) + 2;
-        tot += 4 * G * G * G;
-    }
-    const size_t G0 = (size_t)n + 2;
-    return tot + 2 * G0 * G0 * G0;
-}
-// two result words follow the arrays: relative residual and cycle count
-constexpr size_t NOALLOC_OUT_DOUBLES = 2;
-constexpr size_t NOALLOC_SCRATCH_DOUBLES = noalloc_level_doubles(NOALLOC_MAX_N) + NOALLOC_OUT_DOUBLES;
+template <int TOP>
+__host__ __device__ constexpr int noalloc_ctas() { return TOP >= 5 ? 8 : 1; }
 
-static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_SCRATCH_DOUBLES];
-
-// level arrays of an n^3 base grid laid out from the start of the scratch
-__host__ __device__ inline MgData noalloc_layout(double *s, int n, double h) {
-    MgData d;
-    for (int m = 0; m < MG_MAXLEV; m++) d.U[m] = d.RES[m] = d.RHS[m] = d.RHO[m] = nullptr;
-    int MMax = 0;
-    while ((1 << MMax) < n) MMax++;
-    for (int m = 0; m <= MMax; m++) {
-        const size_t G = (size_t)(n >> m) + 2, V = G * G * G;
-        d.U[m] = s; s += V;
-        d.RES[m] = s; s += V;
-        d.RHS[m] = s; s += V;
-        d.RHO[m] = s; s += V;
-    }
-    const size_t G0 = (size_t)n + 2, V0 = G0 * G0 * G0;
-    d.SRC = s; s += V0;
-    d.PSI = s;
-    d.N = n;
-    d.MMax = MMax;
-    d.hbase = h;
-    d.periodic = 1;
-    d.zbc = 0;
-    for (int f = 0; f < 6; f++) d.touch[f] = 0;   // periodic: no face touches a physical boundary
-    return d;
-}
-
-// One CTA.  rho and psi are dense n^3 arrays, x fastest.  Solves
+// rho and psi are dense n^3 arrays, x fastest, n = 2^TOP.  Solves
 // lap(psi) = four_pi_G * (rho - mean rho) on the periodic grid of cell width
 // h: psi starts at zero; each cycle forms the residual (mg_poisson.F90:5-28),
 // solves for the correction with mg_lin and adds it (mg.F90:62-90), until
 // max|residual| <= rel_tol * max|four_pi_G (rho - mean)| or max_cycles.
-__global__ void __launch_bounds__(1024) k_mg_uniform_noalloc(MgData d, const double *__restrict__ rho,
-                                                             double *__restrict__ psi, double four_pi_G,
-                                                             double rel_tol, int max_cycles, double *out,
-                                                             int64_t clear_doubles) {
-    __shared__ double sh[32];
-    __shared__ double wsum[32];
-    const int n = d.N, G = n + 2, n3 = n * n * n;
-    // one CTA, every level in the scratch array (global memory)
-    MgRun r;
-    r.rank = 0;
-    r.nct = 1;
-    r.wide_min = 1 << 30;
-    r.smem_from = d.MMax + 1;
-    r.pending = false;
-    r.mirror = nullptr;
-    r.slot = nullptr;
-    // every array read below starts at zero (U, RES, RHS, RHO of all levels, SRC, PSI)
-    for (int64_t t = threadIdx.x; t < clear_doubles; t += blockDim.x) d.U[0][t] = 0.0;
+template <int TOP>
+__global__ void __launch_bounds__(512, 1) k_mgs_uniform_noalloc(const double *__restrict__ rho, double *__restrict__ psi,
+                                                                double h, double four_pi_G, double rel_tol,
+                                                                int max_cycles, double *out) {
+    constexpr int C = noalloc_ctas<TOP>();
+    using M = Mgs<TOP, C, kMgPeriodic>;
+    __shared__ typename M::Tables tab;
+    __shared__ double red[32], slot, wsum[32];
+    constexpr int N3 = 1 << (3 * TOP), VOL = M::vol(TOP);
+    double *const sm = M::sm();
+    const int tid = threadIdx.x, rank = C > 1 ? mg_cluster_rank() : 0, first = rank * VOL;
+    const typename M::Ctx x{&tab, rank};
+    M::fill_tables(tab, h);
+    // Mean of rho, in every CTA (rho is at most 256 KB, from L2): 1024 partial
+    // sums in cell order, two per thread, then a fixed tree over each 32 and
+    // the 32 results in order.
+    //
     // A NaN or Inf density would make the mean and every source value NaN;
     // max|source| would then stay 0 (NaN fails every comparison) and the
     // loop would stop at once with psi = 0 reported as converged.  Refuse
     // it instead: psi is set to NaN everywhere and the result words carry a
     // cycle count of -1, which the host turns into SFM_ENONFINITE.
     int bad = 0;
-    for (int c = threadIdx.x; c < n3; c += blockDim.x) bad |= !isfinite(rho[c]);
+#pragma unroll 1
+    for (int half = 0; half < 2; half++) {
+        double s = 0.0;
+        for (int c = tid + 512 * half; c < N3; c += 1024) {
+            const double v = rho[c];
+            bad |= !isfinite(v);
+            s = s + v;
+        }
+        for (int o = 16; o > 0; o >>= 1) s = s + __shfl_down_sync(0xffffffffu, s, o);
+        if ((tid & 31) == 0) wsum[16 * half + (tid >> 5)] = s;
+    }
     if (__syncthreads_or(bad)) {
-        for (int c = threadIdx.x; c < n3; c += blockDim.x) psi[c] = __longlong_as_double(0x7ff8000000000000LL);
-        if (threadIdx.x == 0) {
+        for (int c = tid; c < VOL; c += 512) psi[first + c] = __longlong_as_double(0x7ff8000000000000LL);
+        if (rank == 0 && tid == 0) {
             out[0] = __longlong_as_double(0x7ff8000000000000LL);
             out[1] = -1.0;
         }
         return;
     }
-    // mean of rho: per-thread sums in cell order, then a fixed tree (deterministic)
-    double s = 0.0;
-    for (int c = threadIdx.x; c < n3; c += blockDim.x) s = s + rho[c];
-    for (int o = 16; o > 0; o >>= 1) s = s + __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = s;
-    __syncthreads();
     double tot = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) tot = tot + wsum[w];
-    const double mean = tot / (double)n3;
+    for (int w = 0; w < 32; w++) tot = tot + wsum[w];
+    const double mean = tot / (double)N3;
     double smax = 0.0;
-    for (int c = threadIdx.x; c < n3; c += blockDim.x) {
-        const double v = four_pi_G * (rho[c] - mean);
-        d.SRC[cidx(G, c % n, (c / n) % n, c / (n * n))] = v;
+    for (int c = tid; c < VOL; c += 512) {
+        const double v = four_pi_G * (rho[first + c] - mean);
+        sm[M::SRC + c] = v;
+        sm[M::PSI + c] = 0.0;
         const double a = fabs(v);
         smax = a > smax ? a : smax;
     }
-    smax = mg_block_max(smax, sh);   // synchronises the CTA
+    M::meet();   // every CTA has started before any reads another's shared memory
+    smax = M::vmax(smax, red, &slot);
     int it = 0;
     double rrel = 0.0;
     for (;;) {
-        mg_resid(r, d, 0, d.RHO[0], d.PSI, d.SRC);
-        double v = 0.0;
-        for (int c = threadIdx.x; c < n3; c += blockDim.x) {
-            const double a = fabs(d.RHO[0][cidx(G, c % n, (c / n) % n, c / (n * n))]);
-            v = a > v ? a : v;
-        }
-        const double rmax = mg_block_max(v, sh);
+        const double rmax = M::vmax(M::defect(x), red, &slot);
         rrel = smax > 0.0 ? rmax / smax : 0.0;
         if (rrel <= rel_tol || it >= max_cycles) break;
-        mg_lin(r, d, sh);
-        mg_addw(r, d, 0, d.PSI, d.U[0]);
+        M::correct(x);
+        M::meet();
         it++;
     }
-    for (int c = threadIdx.x; c < n3; c += blockDim.x) psi[c] = d.PSI[cidx(G, c % n, (c / n) % n, c / (n * n))];
-    if (threadIdx.x == 0) {
+    for (int c = tid; c < VOL; c += 512) psi[first + c] = sm[M::PSI + c];
+    if (rank == 0 && tid == 0) {
         out[0] = rrel;
         out[1] = (double)it;
+    }
+}
+
+// go(kernel, CTAs of the cluster, shared bytes) for n = 2^top
+template <class F>
+inline void noalloc_with(int top, F &&go) {
+    auto one = [&](auto t) {
+        constexpr int TOP = decltype(t)::value, C = noalloc_ctas<TOP>();
+        go(k_mgs_uniform_noalloc<TOP>, C, (int)(Mgs<TOP, C, kMgPeriodic>::total() * sizeof(double)));
+    };
+    switch (top) {
+        case 1: one(std::integral_constant<int, 1>{}); break;
+        case 2: one(std::integral_constant<int, 2>{}); break;
+        case 3: one(std::integral_constant<int, 3>{}); break;
+        case 4: one(std::integral_constant<int, 4>{}); break;
+        default: one(std::integral_constant<int, 5>{}); break;
     }
 }
 

@@ -1531,6 +1531,8 @@ public:
             return g;
         }
     }
+    // the grid of the sweep that relax() launches on level f with the table as
+    // it stands: asked for before a capture, since the query may load the kernel
     template <int N, int SW>
     void bulk_grids_of() {
         (void)bulk_grid<N, SW>();
@@ -2639,9 +2641,9 @@ static int check_device(void) {
     if (cudaGetDeviceCount(&n) != cudaSuccess || n <= 0) return SFM_EDEVICE;
     int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return SFM_EDEVICE;
-    if (prop.major != 10) return SFM_EDEVICE;   // built for sm_100a only
+    int major = 0;   // one attribute: all properties take 2.5 ms
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return SFM_EDEVICE;
+    if (major != 10) return SFM_EDEVICE;   // built for sm_100a only
     return SFM_OK;
 }
 
@@ -3141,20 +3143,26 @@ int sfm_debug_solve(sfm_ctx *c, const double *rho, double *psi, double *g, sfm_s
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
-// sfm_uniform_solve_noalloc: device address of the fixed scratch array,
-// looked up once per device with that device current
+// sfm_uniform_solve_noalloc: set-up once per device, with that device
+// current: address of the result words, shared-memory opt-in of every size's
+// kernel (which also loads them, so that a later call may be captured)
 // ---------------------------------------------------------------------------
 namespace {
 constexpr int kNoallocMaxDevices = 64;
 std::mutex g_noalloc_mu;
 double *g_noalloc_ptr[kNoallocMaxDevices] = {};
 
-int noalloc_scratch(int dev, double **out) {
+int noalloc_setup(int dev, double **out) {
     if (dev < 0 || dev >= kNoallocMaxDevices) return SFM_EDEVICE;
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
     if (!g_noalloc_ptr[dev]) {
         void *p = nullptr;
-        if (cudaGetSymbolAddress(&p, sfm::g_noalloc_scratch) != cudaSuccess || !p) {
+        bool ok = cudaGetSymbolAddress(&p, sfm::g_noalloc_out) == cudaSuccess && p;
+        for (int top = 1; top <= 5; top++)
+            sfm::noalloc_with(top, [&](auto kern, int, int smem) {
+                ok = ok && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+            });
+        if (!ok) {
             cudaGetLastError();
             return SFM_ECUDA;
         }
@@ -3192,13 +3200,26 @@ extern "C" int sfm_uniform_solve_noalloc(const double *d_rho, double *d_psi, int
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return SFM_EDEVICE;
     if (!device_pointer_on(d_rho, dev) || !device_pointer_on(d_psi, dev)) return SFM_EINVAL;
-    double *s = nullptr;
-    rc = noalloc_scratch(dev, &s);
+    double *out = nullptr;
+    rc = noalloc_setup(dev, &out);
     if (rc != SFM_OK) return rc;
-    const sfm::MgData d = sfm::noalloc_layout(s, n, h);
-    double *out = s + sfm::noalloc_level_doubles(sfm::NOALLOC_MAX_N);
-    sfm::k_mg_uniform_noalloc<<<1, 1024, 0, st>>>(d, d_rho, d_psi, four_pi_G, rel_tol, max_cycles, out,
-                                                  (int64_t)sfm::noalloc_level_doubles(n));
+    int top = 1;
+    while ((1 << top) < n) top++;
+    sfm::noalloc_with(top, [&](auto kern, int ctas, int smem) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = ctas;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(ctas);
+        cfg.blockDim = dim3(512);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cfg.attrs = at;
+        cfg.numAttrs = ctas > 1 ? 1 : 0;
+        cudaLaunchKernelEx(&cfg, kern, d_rho, d_psi, h, four_pi_G, rel_tol, max_cycles, out);
+    });
     if (cudaGetLastError() != cudaSuccess) return SFM_ECUDA;
     if (!cycles && !rel_residual) return SFM_OK;
     double hv[2] = {0.0, 0.0};

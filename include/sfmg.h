@@ -272,13 +272,13 @@ int sfm_tune_load(sfm_ctx *c, const char *text);
  * outputs the call then returns SFM_ENONFINITE (*cycles = -1).
  * d_rho and d_psi must be device memory of the current device (or managed
  * memory): anything else returns SFM_EINVAL.
- * Working arrays live in one fixed device array of the library (about
- * 2 MiB, enough for n = 32), cleared by the kernel itself before use, so
- * nothing needs zeroing and nothing carries over between calls.  There is
- * one such array per device: calls on one device whose executions overlap
- * (unordered streams, concurrent host threads) race and give wrong results.
- * The first call on each device looks up the array's address; make it
- * before any stream capture on that device.  Uses the current device. */
+ * Working arrays live in shared memory, so nothing needs zeroing and nothing
+ * carries over between calls.  The two result words behind `cycles` and
+ * `rel_residual` are one pair per device: of calls on one device whose
+ * executions overlap (unordered streams, concurrent host threads), one may
+ * get the other's, so order calls that ask for them.
+ * The first call on each device sets the kernels up; make it before any
+ * stream capture on that device.  Uses the current device. */
 #define SFM_NOALLOC_MAX_N 32
 int sfm_uniform_solve_noalloc(const double *d_rho, double *d_psi, int n, double h, double four_pi_G,
                               double rel_tol, int max_cycles, int *cycles, double *rel_residual,
