@@ -538,6 +538,7 @@ public:
         if (!iterExec) {
             int64_t l0 = launches;
             int save = FmgLevel_fill0;
+            sweep_grids();
             if (cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
                 cudaGetLastError();
                 graphsOff = true;
@@ -1067,7 +1068,6 @@ public:
         d_bad = mem.alloc<int>(1);
         d_err = mem.alloc<int>(1);
         zeroList.push_back({d_err, sizeof(int)});
-        for (int f = 0; f <= FMax; f++) SFM_WITH_N(nf[f], bulk_grids<N>(), (void)0);
         d_mom = mem.alloc<double>(32);
         if (P.bc != SFM_BC_PERIODIC)   // per-cell moment terms of the base level, summed in order
             d_part = mem.alloc<double>((size_t)H.lstart[1] * H.NI * H.NI * H.NI * kMomentTerms);
@@ -1484,7 +1484,7 @@ public:
     // block between ghost refreshes)
     int local_sweeps() const { return sched(kKnobLocalSweeps, 1); }
     // persistent grid of k_relax_bulk<T, N> (N >= 4): every SM filled to the
-    // kernel's occupancy; computed once, at set-up, outside stream capture
+    // kernel's occupancy; computed once per variant, outside stream capture
     // the bulk pipeline serves blocks of 4^3 and up whose stages fit in 220 KB
     // (on 2^3 blocks it measured slower than k_relax_tiled)
     template <int N>
@@ -1534,21 +1534,30 @@ public:
     // the grid of the sweep that relax() launches on level f with the table as
     // it stands: asked for before a capture, since the query may load the kernel
     template <int N, int SW>
-    void bulk_grids_of() {
-        (void)bulk_grid<N, SW>();
-        (void)face_grid<N, 256, SW>();
-        (void)face_grid<N, 288, SW>();
-        (void)face_grid<N, 512, SW>();
-        (void)face_grid<N, 544, SW>();
+    void sweep_grid(int f) {
+        if (!faces_at(f)) {
+            (void)bulk_grid<N, SW>();
+            return;
+        }
+        switch (relax_nt(N, SW > 0)) {
+            case 256: (void)face_grid<N, 256, SW>(); break;
+            case 512: (void)face_grid<N, 512, SW>(); break;
+            case 544: (void)face_grid<N, 544, SW>(); break;
+            default: (void)face_grid<N, 288, SW>(); break;
+        }
     }
     template <int N>
-    void bulk_grids() {   // every variant a solve may launch
-        bulk_grids_of<N, 0>();
+    void sweep_grid_of(int f) {
+        const int sw = fused_at(f) ? local_sweeps() : 0;
         if constexpr (sizeof(T) == 4) {
-            bulk_grids_of<N, 1>();
-            bulk_grids_of<N, 2>();
-            bulk_grids_of<N, 3>();
+            if (sw == 1) return sweep_grid<N, 1>(f);
+            if (sw == 2) return sweep_grid<N, 2>(f);
+            if (sw == 3) return sweep_grid<N, 3>(f);
         }
+        sweep_grid<N, 0>(f);
+    }
+    void sweep_grids() {
+        for (int f = 0; f <= H.FMax; f++) SFM_WITH_N(nf[f], sweep_grid_of<N>(f), (void)0);
     }
     template <int N, int SW>
     void relax_bulk_launch(T *u, const T *rhs, const int32_t *blocks, int nblk, const int32_t *rslot, const double *rb,
