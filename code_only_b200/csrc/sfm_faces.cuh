@@ -155,6 +155,10 @@ __global__ void __launch_bounds__(256) k_faces_of(const T *__restrict__ u, T *__
 // expressions).  Waits are bounded as there.  (Planes read straight from
 // global memory into registers left their latency on the consumers' path:
 // 751 us against 370 us for k_relax_bulk's two fused sweeps on jeans6.)
+// Bound by issue slots and the waits between colours.  56 registers a thread,
+// so that nothing spills: two fused sweeps of 8^3 FP32 blocks at 5 CTAs per
+// SM and 40 registers made the six-level cloud's mixed solve 74.5 ms, at 4
+// CTAs 73.2; with places, planes and stages found by division per tile 75.8.
 // ---------------------------------------------------------------------------
 template <class T, int N>
 struct FacePlan {
@@ -171,7 +175,7 @@ struct FacePlan {
 template <class T, int N, int NT>
 __host__ __device__ constexpr int relax_faces_min_ctas() {
     constexpr int bySmem = (228 * 1024) / (FacePlan<T, N>::SMEM + 4 * 1024);
-    constexpr int byRegs = 65536 / (NT * (sizeof(T) == 4 ? 44 : 56));
+    constexpr int byRegs = 65536 / (NT * 56);
     constexpr int m = bySmem < byRegs ? bySmem : byRegs;
     return m < 1 ? 1 : (m > 2048 / NT ? 2048 / NT : m);
 }
@@ -281,7 +285,6 @@ __global__ void __launch_bounds__(NT, relax_faces_min_ctas<T, N, NT>())
     } else {
         const int ct = tid - 32;   // consumer thread 0..NCT-1
         T mt = (T)0;               // max |resh2| (exact in T; widened once)
-        int it = 0;
         // pair t = ct + x NCT of a tile: block q, cells (2 i2, j, k) and (2 i2 + 1, j, k)
         auto pair_of = [&](int x, int &q, int &i2, int &j, int &k) {
             const int t = ct + x * NCT;
@@ -309,9 +312,25 @@ __global__ void __launch_bounds__(NT, relax_faces_min_ctas<T, N, NT>())
         pair_of(0, q0, i20, j0, k0);
         const int par0 = (j0 + k0 + 1) & 1;   // colour 1's cell of the pair
         Nb n1 = around(i20, j0, k0, par0), n2 = around(i20, j0, k0, 1 - par0);
-        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
-            const int s = it % S;
-            const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], (uint32_t)((it / S) & 1), cpolls));
+        // where the pair goes in the block's planes (-1: not on that axis' planes); one cell in x, both in y and z
+        struct Pl3 { int x, y, z; };
+        auto planes_of = [&](int i2, int j, int k) {
+            Pl3 o;
+            o.x = i2 == 0 ? k * N + j : (i2 == HN - 1 ? NN + k * N + j : -1);
+            o.y = j == 0 ? 2 * NN + k * N + 2 * i2 : (j == N - 1 ? 3 * NN + k * N + 2 * i2 : -1);
+            o.z = k == 0 ? 4 * NN + j * N + 2 * i2 : (k == N - 1 ? 5 * NN + j * N + 2 * i2 : -1);
+            return o;
+        };
+        const Pl3 pl0 = planes_of(i20, j0, k0);
+        uint32_t phase = 0;   // stage s, its phase and the data slot by counting: no divisions per tile
+        int s = -1, slot = -1;
+        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            if (++s == S) {
+                s = 0;
+                phase ^= 1;
+            }
+            if (++slot == 2 * R) slot = 0;
+            const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], phase, cpolls));
             if constexpr (SW == 0) {
                 if (!got) {
                     if (lane == 0) atomicExch(&cab, 1);
@@ -319,7 +338,6 @@ __global__ void __launch_bounds__(NT, relax_faces_min_ctas<T, N, NT>())
                 }
             }
             const int first = tile * BPC;
-            const int slot = it % (2 * R);
             T *const st = ring + s * BPC * BLK;
             auto live = [&](int x) {
                 const int t = ct + x * NCT;
@@ -394,8 +412,12 @@ __global__ void __launch_bounds__(NT, relax_faces_min_ctas<T, N, NT>())
                     else own2[x] = v;
                     if (store) u[(int64_t)bid[slot][q] * V + (o.c + LO)] = v;
                     if (keep) ub[o.c] = v;
-                    const T ar = resh2 < (T)0 ? -resh2 : resh2;
-                    mt = ar > mt ? ar : mt;
+                    if constexpr (sizeof(T) == 4) {
+                        mt = fmaxf(fabsf(resh2), mt);   // one instruction; a NaN leaves mt, as the comparison does
+                    } else {
+                        const T ar = resh2 < (T)0 ? -resh2 : resh2;
+                        mt = ar > mt ? ar : mt;
+                    }
                 }
             };
             if constexpr (SW > 0) {
@@ -433,12 +455,12 @@ __global__ void __launch_bounds__(NT, relax_faces_min_ctas<T, N, NT>())
                 int q, i2, j, k;
                 pair_of(x, q, i2, j, k);
                 const bool one = (j + k) & 1;   // colour 1's cell is the even one
+                const Pl3 pl = ITER == 1 ? pl0 : planes_of(i2, j, k);
                 T *o = fa.out + (int64_t)bid[slot][q] * (6 * NN);
                 const T pr[2] = {one ? own1[x] : own2[x], one ? own2[x] : own1[x]};
-                if (i2 == 0) o[k * N + j] = pr[0];
-                if (i2 == HN - 1) o[NN + k * N + j] = pr[1];
-                if (j == 0 || j == N - 1) vec_store<T, 2>(o + (j == 0 ? 2 : 3) * NN + k * N + 2 * i2, pr);
-                if (k == 0 || k == N - 1) vec_store<T, 2>(o + (k == 0 ? 4 : 5) * NN + j * N + 2 * i2, pr);
+                if (pl.x >= 0) o[pl.x] = i2 == 0 ? pr[0] : pr[1];
+                if (pl.y >= 0) vec_store<T, 2>(o + pl.y, pr);
+                if (pl.z >= 0) vec_store<T, 2>(o + pl.z, pr);
             }
         }
         m = (double)mt;

@@ -24,10 +24,8 @@
 //     before any stream capture on that device.
 //
 // Bound by the serial chain of colour sweeps and transfers (about 400
-// dependent steps a cycle).  A call at n = 32 and rel_tol 1e-10: 2.83 ms with
-// the level arrays in global memory on one CTA of 1024 threads, 0.58 ms here
-// (2.2 ms of the first figure hid the host's 2.5 ms device query, which is
-// gone too; the kernel alone went from 2.1 to 0.55 ms).
+// dependent steps a cycle).  n = 32, rel_tol 1e-10: 2.1 ms with the level
+// arrays in global memory on one CTA of 1024 threads, 0.55 ms here.
 #pragma once
 #include "sfm_mgs.cuh"
 
