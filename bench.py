@@ -397,7 +397,7 @@ def run_ours(args):
         "context_create_s": {"mixed": round(mx["create_s"], 3), "fp64": round(fp["create_s"], 3)},
         "phi_rel_err_mixed_vs_fp64": phi_err,
         "roofline": {
-            "kernel": f"k_relax_bulk<float, {h.ni}>: " + (f"{colours // 2} fused red-black sweep(s)" if colours >= 2
+            "kernel": f"k_relax_faces<float, {h.ni}>: " + (f"{colours // 2} fused red-black sweep(s)" if colours >= 2
                                                           else "one red-black colour") + " over the leaf cells, fmg level 0",
             "bound": "hbm", "achieved": round(achieved, 1) if achieved else None, "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 4) if achieved else None,
