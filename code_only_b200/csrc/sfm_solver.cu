@@ -207,6 +207,11 @@ struct DevMem {
     int64_t bytes = 0;
     cudaError_t err = cudaSuccess;
     uint64_t guard = g_guard_bytes.load();
+    // Uploads and clears are queued here: the context's own stream, which its
+    // set-up waits for before it returns.  On the legacy default stream
+    // nothing would order them before a solve, whose streams may be
+    // non-blocking ones.
+    cudaStream_t stream = nullptr;
     struct Band { unsigned char *lo, *hi; size_t hiLen; };   // the bands below and above one array
     std::vector<Band> bands;
     template <class T>
@@ -220,8 +225,8 @@ struct DevMem {
             if (e != cudaSuccess) { err = e; return nullptr; }
             ptrs.push_back(p);
             unsigned char *base = static_cast<unsigned char *>(p);
-            e = cudaMemset(base, kGuardByte, guard);
-            if (e == cudaSuccess) e = cudaMemset(base + guard + payload, kGuardByte, body - payload + guard);
+            e = cudaMemsetAsync(base, kGuardByte, guard, stream);
+            if (e == cudaSuccess) e = cudaMemsetAsync(base + guard + payload, kGuardByte, body - payload + guard, stream);
             if (e != cudaSuccess) { err = e; return nullptr; }
             bands.push_back({base, base + guard + payload, body - payload + guard});
             bytes += (int64_t)payload;
@@ -250,10 +255,20 @@ struct DevMem {
     T *upload(const std::vector<T> &v) {
         T *p = alloc<T>(v.size());
         if (p && !v.empty()) {
-            cudaError_t e = cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+            // pageable memory: v may go as soon as the call returns
+            cudaError_t e = cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, stream);
             if (e != cudaSuccess) err = e;
         }
         return p;
+    }
+    void clear(void *p, size_t bytes) {
+        if (!p) return;
+        cudaError_t e = cudaMemsetAsync(p, 0, bytes, stream);
+        if (e != cudaSuccess) err = e;
+    }
+    void wait() {   // for what has been queued
+        cudaError_t e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) err = e;
     }
     void release() {
         for (void *p : ptrs) cudaFree(p);
@@ -817,6 +832,7 @@ public:
         P = *p;
         if (cudaStreamCreateWithFlags(&own_, cudaStreamNonBlocking) != cudaSuccess) return SFM_ECUDA;
         st_ = own_;
+        mem.stream = own_;
         {
             int dev = 0, sms = 148;
             cudaGetDevice(&dev);
@@ -1047,8 +1063,7 @@ public:
             const size_t nn = facesOk && face_edge(nf[f]) ? (size_t)nf[f] * nf[f] : 0;
             for (auto &b : faceBuf) b.push_back(nn ? mem.alloc<T>((size_t)nb * 6 * nn) : nullptr);
             cfBuf.push_back(nn ? mem.alloc<T>((size_t)(nReflux + 1) * nn) : nullptr);   // and a plane of zeros
-            if (nn && cfBuf.back() && cudaMemset(cfBuf.back() + (size_t)nReflux * nn, 0, nn * sizeof(T)) != cudaSuccess)
-                mem.err = cudaErrorUnknown;
+            if (nn && cfBuf.back()) mem.clear(cfBuf.back() + (size_t)nReflux * nn, nn * sizeof(T));
             facePar.push_back(-1);
         }
         if (facesOk && tfL.empty() && (H.NI == 4 || H.NI == 8 || H.NI == 16)) {
@@ -1121,6 +1136,7 @@ public:
             zeroList.push_back({mg.PSI, V0 * sizeof(double)});
             mgs_init();
         }
+        mem.wait();
         if (mem.err != cudaSuccess) {
             last_error = cudaGetErrorString(mem.err);
             return mem.err == cudaErrorMemoryAllocation ? SFM_ENOMEM : SFM_ECUDA;
@@ -2420,6 +2436,7 @@ public:
         aPart = mem.alloc<double>((size_t)std::max<int64_t>(tfLOff[H.nlev], 1) * 25);
         aBeta = mem.alloc<double>(32);
         aDot = mem.alloc<double>(8);
+        mem.wait();
         if (mem.err != cudaSuccess) {
             last_error = cudaGetErrorString(mem.err);
             return mem.err == cudaErrorMemoryAllocation ? SFM_ENOMEM : SFM_ECUDA;
