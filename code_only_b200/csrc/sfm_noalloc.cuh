@@ -17,9 +17,10 @@
 //   - n (cells per edge) is a power of two, 2 <= n <= SFM_NOALLOC_MAX_N (32);
 //   - no state carries over from one call to the next;
 //   - the two result words (residual, cycle count) are one pair per device
-//     and loaded library: of two calls on the same device whose executions
-//     overlap, the host outputs of either may be the other's.  Order calls
-//     that ask for host outputs on one stream or with events;
+//     and loaded library, written only by calls that ask for host outputs: of
+//     two such calls on the same device whose executions overlap, the host
+//     outputs and the status of either may be the other's.  Order calls that
+//     ask for host outputs on one stream or with events;
 //   - the first call on each device does the set-up; make that first call
 //     before any stream capture on that device.
 //
@@ -42,6 +43,7 @@ __host__ __device__ constexpr int noalloc_ctas() { return TOP >= 5 ? 8 : 1; }
 // h: psi starts at zero; each cycle forms the residual (mg_poisson.F90:5-28),
 // solves for the correction with mg_lin and adds it (mg.F90:62-90), until
 // max|residual| <= rel_tol * max|four_pi_G (rho - mean)| or max_cycles.
+// out: the result words, or null where the call asks for none.
 template <int TOP>
 __global__ void __launch_bounds__(512, 1) k_mgs_uniform_noalloc(const double *__restrict__ rho, double *__restrict__ psi,
                                                                 double h, double four_pi_G, double rel_tol,
@@ -78,7 +80,7 @@ __global__ void __launch_bounds__(512, 1) k_mgs_uniform_noalloc(const double *__
     }
     if (__syncthreads_or(bad)) {
         for (int c = tid; c < VOL; c += 512) psi[first + c] = __longlong_as_double(0x7ff8000000000000LL);
-        if (rank == 0 && tid == 0) {
+        if (out && rank == 0 && tid == 0) {
             out[0] = __longlong_as_double(0x7ff8000000000000LL);
             out[1] = -1.0;
         }
@@ -108,7 +110,7 @@ __global__ void __launch_bounds__(512, 1) k_mgs_uniform_noalloc(const double *__
         it++;
     }
     for (int c = tid; c < VOL; c += 512) psi[first + c] = sm[M::PSI + c];
-    if (rank == 0 && tid == 0) {
+    if (out && rank == 0 && tid == 0) {
         out[0] = rrel;
         out[1] = (double)it;
     }

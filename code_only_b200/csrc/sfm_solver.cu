@@ -3244,7 +3244,8 @@ extern "C" int sfm_uniform_solve_noalloc(const double *d_rho, double *d_psi, int
         cfg.stream = st;
         cfg.attrs = at;
         cfg.numAttrs = ctas > 1 ? 1 : 0;
-        cudaLaunchKernelEx(&cfg, kern, d_rho, d_psi, h, four_pi_G, rel_tol, max_cycles, out);
+        cudaLaunchKernelEx(&cfg, kern, d_rho, d_psi, h, four_pi_G, rel_tol, max_cycles,
+                           cycles || rel_residual ? out : nullptr);
     });
     if (cudaGetLastError() != cudaSuccess) return SFM_ECUDA;
     if (!cycles && !rel_residual) return SFM_OK;

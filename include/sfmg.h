@@ -274,9 +274,10 @@ int sfm_tune_load(sfm_ctx *c, const char *text);
  * memory): anything else returns SFM_EINVAL.
  * Working arrays live in shared memory, so nothing needs zeroing and nothing
  * carries over between calls.  The two result words behind `cycles` and
- * `rel_residual` are one pair per device: of calls on one device whose
- * executions overlap (unordered streams, concurrent host threads), one may
- * get the other's, so order calls that ask for them.
+ * `rel_residual` are one pair per device, written only by calls that ask for
+ * them: of such calls on one device whose executions overlap (unordered
+ * streams, concurrent host threads), one may get the other's outputs and
+ * status, so order calls that ask.
  * The first call on each device sets the kernels up; make it before any
  * stream capture on that device.  Uses the current device. */
 #define SFM_NOALLOC_MAX_N 32
