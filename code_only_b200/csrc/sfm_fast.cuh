@@ -493,9 +493,7 @@ __device__ __noinline__ T ghost_cf_face(const T *u, const int8_t *oct, int X, in
 // The remaining CTAs take the general items.
 constexpr int kGhostWarps = 8;   // blocks per sweep CTA (one per warp)
 template <int N>
-__host__ __device__ constexpr int ghost_sweep_ctas(int nblk) {
-    return (nblk + kGhostWarps - 1) / kGhostWarps;
-}
+__host__ __device__ constexpr int ghost_sweep_ctas(int nblk) { return (nblk + kGhostWarps - 1) / kGhostWarps; }
 template <int N>
 __host__ __device__ constexpr int ghost_general_ctas(int items) {
     return (int)(((int64_t)items * N + 255) / 256);   // N cells per item (corners use the first)
@@ -861,12 +859,10 @@ __host__ __device__ constexpr int relax_bulk_min_ctas() {
                ? (228 * 1024) / (BulkPlan<T, N>::SMEM + 1024)
                : (2048 / NT < 8 ? 2048 / NT : 8);
 }
-// threads of k_relax_bulk: warp 0 produces, the others consume.  A 16^3
-// block's stages allow only one or two CTAs per SM, so those CTAs get 15
-// consumer warps instead of 7.
-// (the default; the autotuner may choose the other count per block edge)
-template <int N>
-__host__ __device__ constexpr int relax_bulk_threads() { return N >= 16 ? 512 : 256; }
+// NT threads: warp 0 produces, the others consume.  A 16^3 block's stages
+// allow only one or two CTAs per SM, so those CTAs get 15 consumer warps by
+// default instead of 7; the autotuner may choose another count per block edge
+// (Solver::relax_nt).
 //
 // SW > 0 (a choice of the mixed path's schedule, never of the FP64 path):
 // SW full red-black sweeps of every staged block in one pass -- each
@@ -879,7 +875,7 @@ __host__ __device__ constexpr int relax_bulk_threads() { return N >= 16 ? 512 : 
 // skips the first colour and still reaches the tile's first barrier, which
 // ORs the failures: every consumer warp leaves after it, so none waits at a
 // barrier for one that has gone.  SW = 0: the one colour `ipass`.
-template <class T, int N, int NT = relax_bulk_threads<N>(), int SW = 0>
+template <class T, int N, int NT, int SW>
 __global__ void __launch_bounds__(NT, relax_bulk_min_ctas<T, N, NT>())
     k_relax_bulk(T *__restrict__ u, const T *__restrict__ rhs,
                                                     const int32_t *__restrict__ blocks, int nblk,

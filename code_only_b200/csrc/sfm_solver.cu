@@ -291,6 +291,7 @@ public:
     virtual int fmg_levels() const = 0;
     virtual void set_wait_polls(uint32_t polls) = 0;
     virtual void set_ghost_merge(bool on) = 0;
+    virtual int smoother_threads(int f, bool fused) const = 0;
     virtual void set_serial_relax(bool on) = 0;
     virtual int autotune(int reps, const double *d_rho) = 0;
     virtual std::string tune_text() const = 0;
@@ -381,8 +382,8 @@ public:
     int *d_err = nullptr;                  // set by a device wait that gave up
     uint32_t waitPolls = kWaitPolls;       // poll limit of the smoother's stage waits (tests lower it)
     int nSM = 148;
-    int bulkGrid[5][4] = {};               // persistent CTAs of k_relax_bulk, by log2(N), SW
-    int faceGrid[5][4][4] = {};            // of k_relax_faces, by log2(N), CTA size, SW
+    int bulkGrid[5][4][4] = {};            // persistent CTAs of k_relax_bulk, by log2(N), CTA size, SW
+    int faceGrid[5][4][4] = {};            // of k_relax_faces, likewise
     double *d_mom = nullptr, *d_part = nullptr, *d_psum = nullptr;
     int *d_mgit = nullptr;
     // base grid
@@ -725,13 +726,17 @@ public:
                 const bool fused = kind == 1;
                 if (fused && sizeof(T) != 4) continue;
                 float best = std::numeric_limits<float>::max();
-                int pick = relax_nt(n, fused);
+                int pick = relax_nt(f, fused);
                 for (int nt : kRelaxNT) {
-                    if (!faces_at(f)) break;   // k_relax_bulk has one CTA size
                     tune.set(kKnobRelaxThreads, (int)sizeof(T), n, -1, kind, nt);
                     const float t = time_min([&] {
-                        for (int ipass = 1; ipass <= (fused ? 1 : 2); ipass++)
-                            relax_faces_launch(U[f], RHS[f], f, ipass, d_max, fused ? 1 : 0, false);
+                        for (int ipass = 1; ipass <= (fused ? 1 : 2); ipass++) {
+                            if (faces_at(f))
+                                relax_faces_launch(U[f], RHS[f], f, ipass, d_max, fused ? 1 : 0, false);
+                            else
+                                relax_launch(U[f], RHS[f], d_leaves, nLeaves, d_rslot, rbuf[f], f, ipass, d_max,
+                                             fused ? 1 : 0);
+                        }
                     }, reps);
                     if (t < best) { best = t; pick = nt; }
                 }
@@ -1060,7 +1065,7 @@ public:
         for (int f = 0; f <= FMax; f++) {
             U.push_back(fieldT(f)); RES.push_back(fieldT(f)); RHS.push_back(fieldT(f)); RHO.push_back(fieldT(f));
             rbuf.push_back(mem.alloc<double>((size_t)std::max(nSlots, 1) * nf[f] * nf[f]));
-            const size_t nn = facesOk && face_edge(nf[f]) ? (size_t)nf[f] * nf[f] : 0;
+            const size_t nn = facesOk && bulk_edge(nf[f]) ? (size_t)nf[f] * nf[f] : 0;
             for (auto &b : faceBuf) b.push_back(nn ? mem.alloc<T>((size_t)nb * 6 * nn) : nullptr);
             cfBuf.push_back(nn ? mem.alloc<T>((size_t)(nReflux + 1) * nn) : nullptr);   // and a plane of zeros
             if (nn && cfBuf.back()) mem.clear(cfBuf.back() + (size_t)nReflux * nn, nn * sizeof(T));
@@ -1216,13 +1221,13 @@ public:
         d_child = mem.upload(std::vector<int32_t>(H.child.begin(), H.child.end()));
         d_cf = mem.upload(items);
     }
-    // block edges the plane exchange serves: those of the bulk-copy sweeps
-    static bool face_edge(int n) {
+    // block edges of the bulk-copy sweeps, which are those the plane exchange serves
+    static bool bulk_edge(int n) {
         bool ok = false;
         SFM_WITH_N(n, ok = bulk_ok<N>(), ok = false)
         return ok;
     }
-    bool faces_at(int f) const { return facesOk && !serialRelax && face_edge(nf[f]); }
+    bool faces_at(int f) const { return facesOk && !serialRelax && bulk_edge(nf[f]); }
     FaceArgs<T> face_args(int f, bool zero) const {
         const int p = facePar[f] < 0 ? 0 : facePar[f];
         return FaceArgs<T>{faceBuf[p][f], faceBuf[1 - p][f], cfBuf[f], cfBuf[f] + (size_t)nReflux * nf[f] * nf[f], d_fsrc,
@@ -1527,13 +1532,13 @@ public:
     }
     template <int N>
     static constexpr int log2_edge() { return N >= 16 ? 4 : (N >= 8 ? 3 : 2); }   // capped
-    template <int N, int SW>
+    template <int N, int NT, int SW>
     int bulk_grid() {   // k_relax_bulk
         if constexpr (!bulk_ok<N>()) {
             return 0;
         } else {
-            int &g = bulkGrid[log2_edge<N>()][SW];
-            if (!g) g = resident(k_relax_bulk<T, N, relax_bulk_threads<N>(), SW>, relax_bulk_threads<N>(), BulkPlan<T, N>::SMEM);
+            int &g = bulkGrid[log2_edge<N>()][nt_index<NT>()][SW];
+            if (!g) g = resident(k_relax_bulk<T, N, NT, SW>, NT, BulkPlan<T, N>::SMEM);
             return g;
         }
     }
@@ -1547,20 +1552,25 @@ public:
             return g;
         }
     }
+    // go(NT as a constant) for the CTA size of the smoother on level f
+    template <class F>
+    void with_relax_nt(int f, bool fused, F &&go) {
+        switch (relax_nt(f, fused)) {
+            case 256: go(std::integral_constant<int, 256>{}); break;
+            case 288: go(std::integral_constant<int, 288>{}); break;
+            case 512: go(std::integral_constant<int, 512>{}); break;
+            default: go(std::integral_constant<int, 544>{}); break;
+        }
+    }
     // the grid of the sweep that relax() launches on level f with the table as
     // it stands: asked for before a capture, since the query may load the kernel
     template <int N, int SW>
     void sweep_grid(int f) {
-        if (!faces_at(f)) {
-            (void)bulk_grid<N, SW>();
-            return;
-        }
-        switch (relax_nt(N, SW > 0)) {
-            case 256: (void)face_grid<N, 256, SW>(); break;
-            case 512: (void)face_grid<N, 512, SW>(); break;
-            case 544: (void)face_grid<N, 544, SW>(); break;
-            default: (void)face_grid<N, 288, SW>(); break;
-        }
+        with_relax_nt(f, SW > 0, [&](auto nt) {
+            constexpr int NT = decltype(nt)::value;
+            if (faces_at(f)) (void)face_grid<N, NT, SW>();
+            else (void)bulk_grid<N, NT, SW>();
+        });
     }
     template <int N>
     void sweep_grid_of(int f) {
@@ -1578,27 +1588,24 @@ public:
     template <int N, int SW>
     void relax_bulk_launch(T *u, const T *rhs, const int32_t *blocks, int nblk, const int32_t *rslot, const double *rb,
                            int f, int ipass, unsigned long long *out) {
-        launch_pdl(k_relax_bulk<T, N, relax_bulk_threads<N>(), SW>,
-                   (unsigned)std::min((nblk + Tile<N>::BPC - 1) / Tile<N>::BPC, bulk_grid<N, SW>()),
-                   relax_bulk_threads<N>(), BulkPlan<T, N>::SMEM, u, rhs, blocks, nblk, d_h0, d_level, rslot, rb, f, ipass,
-                   out, d_err, waitPolls);
-    }
-    template <int N, int NT, int SW>
-    void relax_faces_nt(T *u, const T *rhs, int f, int ipass, unsigned long long *out, bool zero) {
-        launch_pdl(k_relax_faces<T, N, NT, SW>,
-                   (unsigned)std::min((nLeaves + Tile<N>::BPC - 1) / Tile<N>::BPC, face_grid<N, NT, SW>()), NT,
-                   FacePlan<T, N>::SMEM, u, rhs, (const int32_t *)d_leaves, nLeaves, (const double *)d_h0,
-                   (const int32_t *)d_level, (const int32_t *)d_rslot, (const double *)rbuf[f], face_args(f, zero), f,
-                   ipass, out, d_err, waitPolls);
+        with_relax_nt(f, SW > 0, [&](auto nt) {
+            constexpr int NT = decltype(nt)::value;
+            launch_pdl(k_relax_bulk<T, N, NT, SW>,
+                       (unsigned)std::min((nblk + Tile<N>::BPC - 1) / Tile<N>::BPC, bulk_grid<N, NT, SW>()), NT,
+                       BulkPlan<T, N>::SMEM, u, rhs, blocks, nblk, d_h0, d_level, rslot, rb, f, ipass, out, d_err,
+                       waitPolls);
+        });
     }
     template <int N, int SW>
     void relax_faces_sw(T *u, const T *rhs, int f, int ipass, unsigned long long *out, bool zero) {
-        switch (relax_nt(N, SW > 0)) {
-            case 256: relax_faces_nt<N, 256, SW>(u, rhs, f, ipass, out, zero); break;
-            case 512: relax_faces_nt<N, 512, SW>(u, rhs, f, ipass, out, zero); break;
-            case 544: relax_faces_nt<N, 544, SW>(u, rhs, f, ipass, out, zero); break;
-            default: relax_faces_nt<N, 288, SW>(u, rhs, f, ipass, out, zero); break;
-        }
+        with_relax_nt(f, SW > 0, [&](auto nt) {
+            constexpr int NT = decltype(nt)::value;
+            launch_pdl(k_relax_faces<T, N, NT, SW>,
+                       (unsigned)std::min((nLeaves + Tile<N>::BPC - 1) / Tile<N>::BPC, face_grid<N, NT, SW>()), NT,
+                       FacePlan<T, N>::SMEM, u, rhs, (const int32_t *)d_leaves, nLeaves, (const double *)d_h0,
+                       (const int32_t *)d_level, (const int32_t *)d_rslot, (const double *)rbuf[f], face_args(f, zero), f,
+                       ipass, out, d_err, waitPolls);
+        });
     }
     // the sweep over all leaves with planes: one colour, or sw > 0 full sweeps
     void relax_faces_launch(T *u, const T *rhs, int f, int ipass, unsigned long long *out, int sw, bool zero) {
@@ -1617,11 +1624,16 @@ public:
         SFM_WITH_N(nf[f], go(std::integral_constant<int, N>{}), (void)0)
         ++launches;
     }
-    // CTA size of k_relax_faces at block edge n, two-launch sweep (tune key
-    // kind -1) or fused sweeps (kind 1); by default the consumer warps divide
-    // a tile's cell pairs evenly (8 warps for 256 pairs, 16 for 2048)
-    int relax_nt(int n, bool fused) const {
-        return tune.get(kKnobRelaxThreads, (int)sizeof(T), n, -1, fused ? 1 : -1, n >= 16 ? 544 : 288);
+    // CTA size of level f's smoother, two-launch sweep (tune key kind -1) or
+    // fused sweeps (kind 1).  By default k_relax_faces' consumer warps divide
+    // a tile's cell pairs evenly (8 warps for 256 pairs, 16 for 2048), and
+    // k_relax_bulk has 7 and 15 of them (sfm_fast.cuh).
+    int relax_nt(int f, bool fused) const {
+        const int n = nf[f], own = n >= 16 ? 512 : 256;
+        return tune.get(kKnobRelaxThreads, (int)sizeof(T), n, -1, fused ? 1 : -1, faces_at(f) ? own + 32 : own);
+    }
+    int smoother_threads(int f, bool fused) const override {
+        return f >= 0 && f <= H.FMax && bulk_edge(nf[f]) ? relax_nt(f, fused) : 0;
     }
     template <int N>
     void relax_dispatch(T *u, const T *rhs, const int32_t *blocks, int nblk, const int32_t *rslot, const double *rb,
@@ -3136,6 +3148,14 @@ int sfm_debug_set_ghost_merge(sfm_ctx *c, int on) {
     if (!c || !c->s) return SFM_EINVAL;
     c->s->set_ghost_merge(on != 0);
     return SFM_OK;
+}
+
+// Test hook (not part of include/sfmg.h): threads of the CTAs that sweep fmg
+// level f with the tuning table as it stands, fused or one colour per launch;
+// 0 where the level has no bulk-copy smoother.
+int sfm_debug_smoother_threads(const sfm_ctx *c, int f, int fused) {
+    if (!c || !c->s) return SFM_EINVAL;
+    return c->s->smoother_threads(f, fused != 0);
 }
 
 // Test hook (not part of include/sfmg.h): like sfm_solve on host arrays, but

@@ -2,12 +2,15 @@
 expressions in the same order, so a tuned solve must be bit-identical to the
 untuned one (and, in FP64, to the oracle); the table survives a save/load
 round trip and an empty table restores the defaults."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from code_only_b200 import abi, workloads as w
 from code_only_b200.solver import FMGPoisson, SFMError
 from tests.oracle_lib import oracle_solve
+from tests.test_gpu_planes import face_nested
 
 pytestmark = pytest.mark.gpu
 
@@ -138,6 +141,44 @@ def test_smoother_cta_sizes_are_bitwise(name, nt):
         s.load_tune_table(fused + "".join(f"relax_threads 4 {e} -1 {k} {nt}\n" for e in edges for k in (-1, 1)))
         psi_b, g_b, _ = s.solve(rho)
     assert np.array_equal(psi_a, psi_b) and np.array_equal(g_a, g_b)
+
+
+# boxes whose sweeps exchange planes, and those that keep the ghost passes
+SMOOTHER_CASES = {
+    "planes": (lambda: w.small_periodic(2, 8, 3, 1), w.gaussian_peak, abi.SFM_BC_PERIODIC, 32),
+    "passes_zmirror": (lambda: w.mirror_sphere(3, 8, 3), w.wide_sphere, abi.SFM_BC_ZMIRROR, 0),
+    "passes_face_nested": (lambda: face_nested(8), w.gaussian_peak, abi.SFM_BC_PERIODIC, 0),
+    "passes_zmirror_ni16": (lambda: w.mirror_sphere(2, 16, 2), w.wide_sphere, abi.SFM_BC_ZMIRROR, 0),
+}
+
+
+@pytest.mark.parametrize("prec", [abi.SFM_PREC_FP64, abi.SFM_PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("name", list(SMOOTHER_CASES))
+def test_smoother_launches_the_tables_cta_size(name, prec):
+    """relax_threads sets the CTA size of whichever smoother serves a level,
+    with planes or with ghost passes, and never a result bit."""
+    mk, fn, bc, extra = SMOOTHER_CASES[name]
+    h = mk()
+    p = abi.default_params(bc, rel_tol=1e-10, max_outer=40, precision=prec, zero_mean=int(bc == abi.SFM_BC_PERIODIC))
+    rho = w.block_field(h, p.ngh_io, fn)
+    elem, kinds = (8, (-1,)) if prec == abi.SFM_PREC_FP64 else (4, (-1, 1))
+    fused = "" if prec == abi.SFM_PREC_FP64 else f"fused_sweeps 4 {h.ni} -1 -1 3\n"
+    with FMGPoisson(h, params=p) as s:
+        lib = s.lib
+        lib.sfm_debug_smoother_threads.argtypes = [C.c_void_p, C.c_int, C.c_int]
+
+        def threads():
+            return [lib.sfm_debug_smoother_threads(s.ctx, f, int(k > 0)) for f in range(h.ni.bit_length() - 2) for k in kinds]
+
+        edges = [h.ni >> f for f in range(h.ni.bit_length() - 2)]   # down to 4
+        assert threads() == [(512 if e >= 16 else 256) + extra for e in edges for _ in kinds]
+        s.load_tune_table(fused)
+        psi, g, _ = s.solve(rho)
+        for nt in (256, 288, 512, 544):
+            s.load_tune_table(fused + "".join(f"relax_threads {elem} {e} -1 {k} {nt}\n" for e in edges for k in kinds))
+            assert threads() == [nt] * len(threads())
+            psi2, g2, _ = s.solve(rho)
+            assert np.array_equal(psi, psi2) and np.array_equal(g, g2)
 
 
 def test_fused_sweep_is_ignored_in_fp64():
