@@ -583,7 +583,7 @@ public:
     }
 
     ~Solver() override {
-        if (iterExec) cudaGraphExecDestroy(iterExec);
+        drop_graph();
         prof_release();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
@@ -596,23 +596,18 @@ public:
     // a new limit drops it, and the next outer iteration captures again
     void set_serial_relax(bool on) override {
         serialRelax = on;
-        if (iterExec) {
-            cudaGraphExecDestroy(iterExec);
-            iterExec = nullptr;
-        }
+        drop_graph();
     }
     void set_ghost_merge(bool on) override {
         ghostForce = on ? 1 : 0;
-        if (iterExec) {
-            cudaGraphExecDestroy(iterExec);
-            iterExec = nullptr;
-        }
+        drop_graph();
     }
     // -----------------------------------------------------------------
     // Autotuner: times every candidate of every knob in use on this
     // context's hierarchy (each candidate `reps` times after one warm-up
     // launch, CUDA events on the context's stream, minimum kept) and keeps
-    // the fastest in the table.  All candidates give bit-identical fields,
+    // the fastest in the table; a kernel that this context's solves do not
+    // launch is not timed and gets no row.  All candidates give bit-identical fields,
     // so the choice never changes a result; the reference's sweep counts and
     // coarse-level cutoff (fmg.F90:280-288, mg.F90:50-52, vmg.F90:85-91) are
     // not knobs, since they change the iterates.
@@ -644,6 +639,62 @@ public:
             tune.set(kKnobGhostFill, (int)sizeof(TT), n, L, sel, t[1] < t[0] ? 1 : 0);
         }
     }
+    // A variant that is faster alone may be slower in a solve, between other
+    // launches: each group of choices (the one-launch fills of an element size
+    // and selection, a smoother's CTA size, a residual's blocks per CTA) goes
+    // back to the default where the whole is at least 0.2% faster with that --
+    // a solve of the caller's density, or without one an outer iteration on
+    // zero fields.  (Repeated solves differ by 0.05%.  On the six-level cloud
+    // in FP64, 512 threads for the sweeps of 8^3 blocks won alone and cost a
+    // solve 154.4 ms against 154.0 with the default 288; the nested boxes'
+    // one-launch fills give a solve 1.1%.)
+    void tune_whole(const double *d_rho, int reps) {
+        auto whole_ms = [&]() -> float {
+            drop_graph();
+            if (!d_rho) {
+                for (auto &z : zeroList) cudaMemsetAsync(z.first, 0, z.second, st_);   // what was timed before left values
+                if (outerPlanes) outer_planes_of();
+                return time_min([&] { outer_iteration(); }, reps);
+            }
+            float best = std::numeric_limits<float>::max();
+            for (int r = 0; r <= reps; r++) {   // the first captures the graph
+                sfm_stats st;
+                const int rc = solve(d_rho, nullptr, nullptr, &st, own_, 0, nullptr);
+                if (r > 0 && (rc == SFM_OK || rc == SFM_ENOTCONVERGED)) best = std::min(best, (float)st.device_ms);
+            }
+            return best;
+        };
+        std::map<TuneTable::Key, std::vector<TuneTable::Key>> groups;
+        for (const auto &e : tune.v) {
+            TuneTable::Key g = e.first;
+            if (std::get<0>(g) == kKnobGhostFill) std::get<2>(g) = std::get<3>(g) = -1;   // all block edges and levels
+            if (e.second != shape_default(e.first)) groups[g].push_back(e.first);
+        }
+        float best = groups.empty() ? 0.0f : whole_ms();
+        for (const auto &g : groups) {
+            const std::map<TuneTable::Key, int> chosen = tune.v;
+            for (const TuneTable::Key &key : g.second) tune.v[key] = shape_default(key);
+            const float t = whole_ms();
+            if (t < 0.998f * best) best = t;
+            else tune.v = chosen;
+        }
+        drop_graph();
+    }
+    // the launch shape without a table (base grid and schedule: as it is in the table)
+    int shape_default(const TuneTable::Key &key) const {
+        switch (std::get<0>(key)) {
+            case kKnobGhostFill: return 0;
+            case kKnobResidBpc: return resid_bpc<8>();
+            case kKnobRelaxThreads:
+                for (int f = 0; f <= H.FMax; f++)
+                    if (nf[f] == std::get<2>(key)) return relax_nt_default(f);
+        }
+        return tune.v.at(key);
+    }
+    void drop_graph() {   // the iteration's graph holds the launches it was captured with
+        if (iterExec) cudaGraphExecDestroy(iterExec);
+        iterExec = nullptr;
+    }
     // Schedule of the mixed path's inner solve (see sfm_tune.h): coordinate
     // descent from the reference schedule over complete solves of the
     // caller's density, keeping a change only when the solve still reaches
@@ -651,10 +702,7 @@ public:
     // least 2% faster.  The FP64 path keeps the reference's schedule.
     int tune_schedule(const double *d_rho, int reps) {
         auto solve_ms = [&](float &ms) -> bool {
-            if (iterExec) {   // the graph holds the old schedule
-                cudaGraphExecDestroy(iterExec);
-                iterExec = nullptr;
-            }
+            drop_graph();   // it holds the old schedule
             sfm_stats st;
             const int rc = solve(d_rho, nullptr, nullptr, &st, own_, 0, nullptr);
             if (rc != SFM_OK || !(st.true_rel_residual <= P.rel_tol) || !st.converged) return false;
@@ -695,10 +743,7 @@ public:
             }
             tune.set(k.knob, 4, H.NI, -1, -1, pick);
         }
-        if (iterExec) {
-            cudaGraphExecDestroy(iterExec);
-            iterExec = nullptr;
-        }
+        drop_graph();
         return SFM_OK;
     }
     int autotune(int reps, const double *d_rho) override {
@@ -743,33 +788,38 @@ public:
                 tune.set(kKnobRelaxThreads, (int)sizeof(T), n, -1, kind, pick);
             }
         }
-        // residual blocks per CTA on 8^3 blocks (inner and outer precision)
-        for (int f = 0; f <= FMax; f++) {
-            if (nf[f] != 8) continue;
-            const int cand[3] = {1, 2, 4};
+        // k_resid_tiled's blocks per CTA on 8^3 blocks, where it runs: the
+        // descent of fmg_lin without planes, the outer residual without
+        // planes, and the reported residual
+        auto tune_resid = [&](int elem, auto &&op) {
             float best = std::numeric_limits<float>::max();
             int pick = 2;
-            for (int c = 0; c < 3; c++) {
-                tune.set(kKnobResidBpc, (int)sizeof(T), 8, -1, -1, cand[c]);
-                const float t = time_min([&] {
+            for (int c : {1, 2, 4}) {
+                tune.set(kKnobResidBpc, elem, 8, -1, -1, c);
+                const float t = time_min(op, reps);
+                if (t < best) { best = t; pick = c; }
+            }
+            tune.set(kKnobResidBpc, elem, 8, -1, -1, pick);
+        };
+        for (int f = 0; f <= FMax; f++) {
+            if (nf[f] != 8) continue;
+            const bool inner = !faces_at(f);
+            if (inner)
+                tune_resid((int)sizeof(T), [&] {
                     FmgLevel_fill0 = f;   // time the residual kernel alone, not its ghost fill
                     resid<T, T, T>(f, RES[f], U[f], RHS[f], false);
-                }, reps);
-                if (t < best) { best = t; pick = cand[c]; }
-            }
-            tune.set(kKnobResidBpc, (int)sizeof(T), 8, -1, -1, pick);
-            if (sizeof(T) != sizeof(double) && f == 0) {
-                best = std::numeric_limits<float>::max();
-                pick = 2;
-                for (int c = 0; c < 3; c++) {
-                    tune.set(kKnobResidBpc, 8, 8, -1, -1, cand[c]);
-                    const float t = time_min([&] {
+                });
+            if (f == 0 && !(inner && sizeof(T) == sizeof(double))) {
+                if (!outerPlanes)
+                    tune_resid(8, [&] {
                         FmgLevel_fill0 = 0;
                         resid<double, double, T>(0, RHO[0], PSI0, SRC0, false);
-                    }, reps);
-                    if (t < best) { best = t; pick = cand[c]; }
-                }
-                tune.set(kKnobResidBpc, 8, 8, -1, -1, pick);
+                    });
+                else if (P.report_residual)
+                    tune_resid(8, [&] {
+                        FmgLevel_fill0 = 0;
+                        resid<double, double, double>(0, RES0d, PHI0, SRC0, false);
+                    });
             }
         }
         // base-grid launch: one CTA or a cluster (same cells, same expressions)
@@ -795,19 +845,19 @@ public:
             }
             tune.set(kKnobBaseCtas, (int)sizeof(T), NBc, -1, -1, pick.nct);
             tune.set(kKnobBaseWide, (int)sizeof(T), NBc, -1, -1, pick.wide);
-        } else if (useSerialMg) {   // k_mgs_cycle: one shape per base grid, recorded as it is
-            tune.set(kKnobBaseCtas, (int)sizeof(T), NBc, -1, -1, mgsTop >= 5 ? 8 : 1);
-            tune.set(kKnobBaseWide, (int)sizeof(T), NBc, -1, -1, 16);
         }
         FmgLevel_fill0 = Undef;
-        if (iterExec) {   // the graph holds the old launch shapes
-            cudaGraphExecDestroy(iterExec);
-            iterExec = nullptr;
-        }
+        wholeArrays = false;
+        drop_graph();   // it holds the old launch shapes
         int rc = check("autotune");
         if (rc == SFM_OK && d_rho && sizeof(T) == 4) {
             rc = tune_schedule(d_rho, std::min(reps, 2));
             if (rc == SFM_OK) rc = check("autotune schedule");
+        }
+        if (rc == SFM_OK) {
+            tune_whole(d_rho, std::min(reps, 2));
+            rc = check("autotune whole");
+            FmgLevel_fill0 = Undef;
         }
         ghostForce = saveForce;
         return rc;
@@ -815,18 +865,12 @@ public:
     std::string tune_text() const override { return tune.text(); }
     bool tune_load(const char *text) override {
         if (!tune.parse(text)) return false;
-        if (iterExec) {
-            cudaGraphExecDestroy(iterExec);
-            iterExec = nullptr;
-        }
+        drop_graph();
         return true;
     }
     void set_wait_polls(uint32_t polls) override {
         waitPolls = polls;
-        if (iterExec) {
-            cudaGraphExecDestroy(iterExec);
-            iterExec = nullptr;
-        }
+        drop_graph();
     }
     int fmg_levels() const override { return H.FMax + 1; }
 
@@ -1628,9 +1672,9 @@ public:
     // fused sweeps (kind 1).  By default k_relax_faces' consumer warps divide
     // a tile's cell pairs evenly (8 warps for 256 pairs, 16 for 2048), and
     // k_relax_bulk has 7 and 15 of them (sfm_fast.cuh).
+    int relax_nt_default(int f) const { return (nf[f] >= 16 ? 512 : 256) + (faces_at(f) ? 32 : 0); }
     int relax_nt(int f, bool fused) const {
-        const int n = nf[f], own = n >= 16 ? 512 : 256;
-        return tune.get(kKnobRelaxThreads, (int)sizeof(T), n, -1, fused ? 1 : -1, faces_at(f) ? own + 32 : own);
+        return tune.get(kKnobRelaxThreads, (int)sizeof(T), nf[f], -1, fused ? 1 : -1, relax_nt_default(f));
     }
     int smoother_threads(int f, bool fused) const override {
         return f >= 0 && f <= H.FMax && bulk_edge(nf[f]) ? relax_nt(f, fused) : 0;
@@ -2285,10 +2329,7 @@ public:
         FmgLevel_fill0 = Undef;
         if (wholeArrays != (stop_stage != 0)) {   // the iteration's graph was captured for the other
             wholeArrays = stop_stage != 0;
-            if (iterExec) {
-                cudaGraphExecDestroy(iterExec);
-                iterExec = nullptr;
-            }
+            drop_graph();
         }
         // fmg_make_physvar
         if (wholeArrays)

@@ -13,13 +13,15 @@
 //   relax_threads threads of the bulk-copy smoother CTA (256, 288, 512 or
 //                 544); key: element size, block edge n, kind -1 for the
 //                 two colour launches, 1 for the fused sweep
-//   resid_bpc     blocks per CTA of the tiled residual (1, 2 or 4);
-//                 key: element size, block edge n
+//   resid_bpc     blocks per CTA of the tiled residual (1, 2 or 4), which
+//                 serves where the plane exchange does not, and the reported
+//                 residual; key: element size, block edge n
 //   base_ctas     CTAs of the base-grid multigrid launch: 1, or a cluster
 //                 of 2, 4, 8 or 16 (sfm_mg.cuh); key: element size, base
 //                 grid cells per edge.  Base grids that k_mgs_cycle serves
 //                 (sfm_mgs.cuh, up to 32^3 cells) have one shape each: the
-//                 entry is kept and not consulted
+//                 tuner gives them no entry, and one in a loaded table is
+//                 kept and not consulted
 //   base_wide     with a cluster, the smallest level (cells per edge: 16,
 //                 32 or 64) whose steps use every CTA; same key
 // and, for the mixed-precision path only (element size 4), the schedule of

@@ -225,7 +225,9 @@ int sfm_info(const sfm_ctx *c, int32_t *fmg_levels, int64_t *device_bytes);
  *
  * sfm_autotune times every launch-shape candidate the context's hierarchy
  * uses (each `reps` times, 1 <= reps <= 100, on the context's own stream and
- * fields; the fields are zeroed first) and keeps the fastest.  With d_rho (a
+ * fields; the fields are zeroed first) and keeps the fastest, unless a whole
+ * solve of d_rho (without d_rho: an outer iteration) is faster with the
+ * built-in choice.  With d_rho (a
  * density in sfm_solve_device's layout, device memory of the context's
  * device) a mixed-precision context also tunes the schedule by complete
  * solves of that density: from the reference's schedule, one knob at a

@@ -10,7 +10,7 @@ import pytest
 from code_only_b200 import abi, workloads as w
 from code_only_b200.solver import FMGPoisson, SFMError
 from tests.oracle_lib import oracle_solve
-from tests.test_gpu_planes import face_nested
+from tests.test_gpu_planes import box, face_nested
 
 pytestmark = pytest.mark.gpu
 
@@ -247,12 +247,39 @@ def test_base_grid_cluster_is_bitwise(name, nct, wide):
     assert np.array_equal(psi, psi2) and np.array_equal(g, g2)
 
 
-def test_autotuned_base_grid_choice_is_recorded():
-    mk, nbase = BASE_CASES["uniform128"]
-    h = mk()
-    p = abi.default_params(abi.SFM_BC_PERIODIC, rel_tol=1e-10, max_outer=30)
+@pytest.mark.parametrize("prec", [abi.SFM_PREC_FP64, abi.SFM_PREC_MIXED], ids=["fp64", "mixed"])
+def test_autotuned_base_grid_choice_is_recorded(prec):
+    """On a base grid of 64^3 cells, which k_mg_cycle serves, the tuner times
+    its shapes and records one."""
+    h = box(32, 4, abi.SFM_BC_PERIODIC)
+    p = abi.default_params(abi.SFM_BC_PERIODIC, rel_tol=1e-10, max_outer=2, precision=prec)
+    elem = 8 if prec == abi.SFM_PREC_FP64 else 4
     with FMGPoisson(h, params=p) as s:
-        s.autotune(2)
+        s.autotune(1)
         lines = s.tune_table().splitlines()
-    assert any(ln.startswith(f"base_ctas 8 {nbase} ") for ln in lines)
-    assert any(ln.startswith(f"base_wide 8 {nbase} ") for ln in lines)
+    assert any(ln.startswith(f"base_ctas {elem} 64 ") for ln in lines)
+    assert any(ln.startswith(f"base_wide {elem} 64 ") for ln in lines)
+
+
+@pytest.mark.parametrize("report", [0, 1])
+@pytest.mark.parametrize("prec", [abi.SFM_PREC_FP64, abi.SFM_PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("name,planes,outer", [("planes", True, True), ("isolated", True, False),
+                                               ("passes_zmirror", False, False)])
+def test_tuner_times_what_the_solve_launches(name, planes, outer, prec, report):
+    """Rows of kernels that a context's solves do not launch are absent: the
+    tiled residual where planes serve (but for the reported residual), and
+    the shapes of k_mg_cycle on a base grid that k_mgs_cycle serves."""
+    mk, fn, bc, _ = (SMOOTHER_CASES | {"isolated": (lambda: w.small_sphere(2, 8, 3, 2), w.softened_sphere,
+                                                    abi.SFM_BC_SPHERE, 0)})[name]
+    h = mk()
+    p = abi.default_params(bc, precision=prec, zero_mean=int(bc == abi.SFM_BC_PERIODIC), report_residual=report)
+    with FMGPoisson(h, params=p) as s:
+        s.autotune(1)
+        rows = {tuple(ln.split()[:3]) for ln in s.tune_table().splitlines()[1:]}
+    elem = "8" if prec == abi.SFM_PREC_FP64 else "4"
+    want = set() if planes else {elem}       # the descent of fmg_lin
+    if not outer or report:                  # the outer residual, the reported one
+        want.add("8")
+    assert {r[1] for r in rows if r[0] == "resid_bpc"} == want
+    assert not any(r[0] in ("base_ctas", "base_wide") for r in rows)
+    assert ("relax_threads", elem, "8") in rows
