@@ -292,7 +292,7 @@ public:
     virtual void set_wait_polls(uint32_t polls) = 0;
     virtual void set_ghost_merge(bool on) = 0;
     virtual int smoother_threads(int f, bool fused) const = 0;
-    virtual void set_serial_relax(bool on) = 0;
+    virtual bool set_serial_relax(bool on) = 0;
     virtual int autotune(int reps, const double *d_rho) = 0;
     virtual std::string tune_text() const = 0;
     virtual bool tune_load(const char *text) = 0;
@@ -356,7 +356,7 @@ public:
     CFItem *d_cf = nullptr;
     std::vector<T *> faceBuf[2], cfBuf;
     std::vector<int> facePar;              // buffer holding U[f]'s planes, -1: neither
-    // the outer residual's (boxes without physical-boundary faces): planes of PSI0
+    // the outer residual's (boxes without physical-boundary faces): planes of PSI0 ([6 nb][n^2], fewer values than RES0d's)
     double *outerPlanes = nullptr, *outerCf = nullptr;
     // whole arrays as the reference leaves them, unread ghost cells and
     // refined blocks included (the debug entry's stage dumps compare them)
@@ -594,9 +594,12 @@ public:
     int64_t guard_violations() const override { return mem.guard_violations(); }
     // the iteration graph holds the kernel parameters it was captured with:
     // a new limit drops it, and the next outer iteration captures again
-    void set_serial_relax(bool on) override {
-        serialRelax = on;
+    bool set_serial_relax(bool on) override {
         drop_graph();
+        for (int f = 0; on && f <= H.FMax; f++)   // the ghost passes' residuals, where planes serve otherwise
+            if (!RES[f]) RES[f] = fieldT(f);
+        serialRelax = on && mem.err == cudaSuccess;
+        return serialRelax == on;
     }
     void set_ghost_merge(bool on) override {
         ghostForce = on ? 1 : 0;
@@ -777,9 +780,9 @@ public:
                     const float t = time_min([&] {
                         for (int ipass = 1; ipass <= (fused ? 1 : 2); ipass++) {
                             if (faces_at(f))
-                                relax_faces_launch(U[f], RHS[f], f, ipass, d_max, fused ? 1 : 0, false);
+                                relax_faces_launch(U[f], RHO[f], f, ipass, d_max, fused ? 1 : 0, false);
                             else
-                                relax_launch(U[f], RHS[f], d_leaves, nLeaves, d_rslot, rbuf[f], f, ipass, d_max,
+                                relax_launch(U[f], RHO[f], d_leaves, nLeaves, d_rslot, rbuf[f], f, ipass, d_max,
                                              fused ? 1 : 0);
                         }
                     }, reps);
@@ -807,7 +810,7 @@ public:
             if (inner)
                 tune_resid((int)sizeof(T), [&] {
                     FmgLevel_fill0 = f;   // time the residual kernel alone, not its ghost fill
-                    resid<T, T, T>(f, RES[f], U[f], RHS[f], false);
+                    resid<T, T, T>(f, RES[f], U[f], RHO[f], false);
                 });
             if (f == 0 && !(inner && sizeof(T) == sizeof(double))) {
                 if (!outerPlanes)
@@ -1104,21 +1107,20 @@ public:
         // ---- fields
         nf.resize(FMax + 1); Gf.resize(FMax + 1); Vf.resize(FMax + 1);
         for (int f = 0; f <= FMax; f++) { nf[f] = H.NI >> f; Gf[f] = nf[f] + 2; Vf[f] = (int64_t)Gf[f] * Gf[f] * Gf[f]; }
-        auto fieldT = [&](int f) { T *p = mem.alloc<T>((size_t)nb * Vf[f]); zeroList.push_back({p, (size_t)nb * Vf[f] * sizeof(T)}); return p; };
         auto fieldD = [&](int f) { double *p = mem.alloc<double>((size_t)nb * Vf[f]); zeroList.push_back({p, (size_t)nb * Vf[f] * sizeof(double)}); return p; };
         for (int f = 0; f <= FMax; f++) {
-            U.push_back(fieldT(f)); RES.push_back(fieldT(f)); RHS.push_back(fieldT(f)); RHO.push_back(fieldT(f));
+            U.push_back(fieldT(f)); RHO.push_back(fieldT(f));
+            // residuals of the descent, and of the corrections of the ascent:
+            // only where the ghost passes serve (and the AMR-level V-cycle's tau)
+            RES.push_back(f == FMax || !faces_at(f) ? fieldT(f) : nullptr);
+            // the finest level's sweeps read RHO (fmg_lin)
+            RHS.push_back(f > 0 ? fieldT(f) : nullptr);
             rbuf.push_back(mem.alloc<double>((size_t)std::max(nSlots, 1) * nf[f] * nf[f]));
             const size_t nn = facesOk && bulk_edge(nf[f]) ? (size_t)nf[f] * nf[f] : 0;
             for (auto &b : faceBuf) b.push_back(nn ? mem.alloc<T>((size_t)nb * 6 * nn) : nullptr);
             cfBuf.push_back(nn ? mem.alloc<T>((size_t)(nReflux + 1) * nn) : nullptr);   // and a plane of zeros
             if (nn && cfBuf.back()) mem.clear(cfBuf.back() + (size_t)nReflux * nn, nn * sizeof(T));
             facePar.push_back(-1);
-        }
-        if (facesOk && tfL.empty() && (H.NI == 4 || H.NI == 8 || H.NI == 16)) {
-            const size_t nn = (size_t)H.NI * H.NI;
-            outerPlanes = mem.alloc<double>((size_t)nb * 6 * nn);
-            outerCf = mem.alloc<double>((size_t)std::max(nReflux, 1) * nn);
         }
         for (int b : leafList) {   // the ordered volume sum of the leaf mean (fmg_data_if.F90:59-77)
             const double hd = H.h0[H.level[b]];
@@ -1127,6 +1129,11 @@ public:
         }
         RUF = fieldT(FMax);
         SRC0 = fieldD(0); PSI0 = fieldD(0); PHI0 = fieldD(0); RES0d = fieldD(0);
+        if (facesOk && tfL.empty() && (H.NI == 4 || H.NI == 8 || H.NI == 16)) {
+            // of the iterations; RES0d holds the residual reported after them
+            outerPlanes = RES0d;
+            outerCf = mem.alloc<double>((size_t)std::max(nReflux, 1) * H.NI * H.NI);
+        }
         d_max = mem.alloc<unsigned long long>(8);
         d_scal = mem.alloc<double>(8);
         d_bad = mem.alloc<int>(1);
@@ -1155,35 +1162,8 @@ public:
                 mg.touch[f] = 0;
                 for (int b = H.lstart[0]; b < H.lstart[1]; b++) mg.touch[f] |= H.touch[6 * b + f];
             }
-            for (int m = 0; m <= MMax; m++) {
-                size_t G = (size_t)(NBc >> m) + 2, V = G * G * G;
-                mg.U[m] = mem.alloc<double>(V); mg.RES[m] = mem.alloc<double>(V);
-                mg.RHS[m] = mem.alloc<double>(V); mg.RHO[m] = mem.alloc<double>(V);
-                for (double *q : {mg.U[m], mg.RES[m], mg.RHS[m], mg.RHO[m]}) zeroList.push_back({q, V * sizeof(double)});
-            }
-            // shared-memory plans of the one-CTA launch and of the cluster
-            // launches (one per wide threshold); opt in to the largest,
-            // whatever the size: static and dynamic together may pass 48 KB
-            size_t most = 0;
-            for (int w : {0, 16, 32, 64}) most = std::max(most, mg_plan(w).bytes);
-            bool optin = cudaFuncSetAttribute(k_mg_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) ==
-                         cudaSuccess;
-            if (!optin) cudaGetLastError();
-            mgSmemOk = optin;
-            if (cudaFuncSetAttribute(k_mg_cycle, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-                cudaGetLastError();
-            const MgPlan one = mg_plan(0);
-            mgSmemFrom = one.from;
-            mgSmemBytes = one.bytes;
-            // which cluster shapes can be resident, asked once here (outside
-            // any stream capture); a table may only pick among these
-            for (int a = 0; a < 5; a++)
-                for (int b = 0; b < 3; b++) mgFits[a][b] = mg_cluster_fits(2 << a, 16 << b);
-            size_t G0 = (size_t)NBc + 2, V0 = G0 * G0 * G0;
-            mg.SRC = mem.alloc<double>(V0); mg.PSI = mem.alloc<double>(V0);
-            zeroList.push_back({mg.SRC, V0 * sizeof(double)});
-            zeroList.push_back({mg.PSI, V0 * sizeof(double)});
             mgs_init();
+            if (mgsTop == 0) mg_init();
         }
         mem.wait();
         if (mem.err != cudaSuccess) {
@@ -1264,6 +1244,13 @@ public:
         d_fsrc = mem.upload(src);
         d_child = mem.upload(std::vector<int32_t>(H.child.begin(), H.child.end()));
         d_cf = mem.upload(items);
+    }
+    // one value per cell, ghosts included, of every block on fmg level f: zero at the start of every solve
+    T *fieldT(int f) {
+        const size_t count = (size_t)H.nb * Vf[f];
+        T *p = mem.alloc<T>(count);
+        if (p) zeroList.push_back({p, count * sizeof(T)});
+        return p;
     }
     // block edges of the bulk-copy sweeps, which are those the plane exchange serves
     static bool bulk_edge(int n) {
@@ -2010,6 +1997,37 @@ public:
         mg_launch(tune.get(kKnobBaseCtas, (int)sizeof(T), NBc, -1, -1, NBc >= 32 && mg_fits(16, 16) ? 16 : 1),
                   tune.get(kKnobBaseWide, (int)sizeof(T), NBc, -1, -1, 16));
         run(OpMgScatter<T>{u, mg.PSI, d_baseIdx, H.ngb[0], H.ngb[1], nf[F], Gf[F], NBc, Vf[F]}, N3);
+    }
+    // k_mg_cycle's level arrays and launch plans
+    void mg_init() {
+        for (int m = 0; m <= mg.MMax; m++) {
+            size_t G = (size_t)(NBc >> m) + 2, V = G * G * G;
+            mg.U[m] = mem.alloc<double>(V); mg.RES[m] = mem.alloc<double>(V);
+            mg.RHS[m] = mem.alloc<double>(V); mg.RHO[m] = mem.alloc<double>(V);
+            for (double *q : {mg.U[m], mg.RES[m], mg.RHS[m], mg.RHO[m]}) zeroList.push_back({q, V * sizeof(double)});
+        }
+        // shared-memory plans of the one-CTA launch and of the cluster
+        // launches (one per wide threshold); opt in to the largest,
+        // whatever the size: static and dynamic together may pass 48 KB
+        size_t most = 0;
+        for (int w : {0, 16, 32, 64}) most = std::max(most, mg_plan(w).bytes);
+        bool optin = cudaFuncSetAttribute(k_mg_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) ==
+                     cudaSuccess;
+        if (!optin) cudaGetLastError();
+        mgSmemOk = optin;
+        if (cudaFuncSetAttribute(k_mg_cycle, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            cudaGetLastError();
+        const MgPlan one = mg_plan(0);
+        mgSmemFrom = one.from;
+        mgSmemBytes = one.bytes;
+        // which cluster shapes can be resident, asked once here (outside
+        // any stream capture); a table may only pick among these
+        for (int a = 0; a < 5; a++)
+            for (int b = 0; b < 3; b++) mgFits[a][b] = mg_cluster_fits(2 << a, 16 << b);
+        size_t G0 = (size_t)NBc + 2, V0 = G0 * G0 * G0;
+        mg.SRC = mem.alloc<double>(V0); mg.PSI = mem.alloc<double>(V0);
+        zeroList.push_back({mg.SRC, V0 * sizeof(double)});
+        zeroList.push_back({mg.PSI, V0 * sizeof(double)});
     }
     // k_mgs_cycle for this base grid: go(kernel, CTAs of the cluster, shared bytes)
     int mgsTop = 0, mgsMode = 0;   // log2 of the base grid's edge (0: k_mg_cycle), MgMode
@@ -3178,8 +3196,8 @@ int sfm_debug_check_guards(sfm_ctx *c, int64_t *bad_bytes) {
 // of a colour depends on another cell of the same colour (race check).
 int sfm_debug_set_serial_relax(sfm_ctx *c, int on) {
     if (!c || !c->s) return SFM_EINVAL;
-    c->s->set_serial_relax(on != 0);
-    return SFM_OK;
+    DeviceGuard dg(c->device);
+    return c->s->set_serial_relax(on != 0) ? SFM_OK : SFM_ENOMEM;
 }
 
 // Test hook (not part of include/sfmg.h): 0 fills every level's ghost

@@ -97,6 +97,36 @@ def test_large_base_levels_match_oracle(nbase):
     check(box(nbase, 4, PER), PER, abi.SFM_PREC_FP64, max_outer=2)
 
 
+# hierarchy, and the device bytes that a context of it held in FP64 and in
+# mixed precision when every sweep had ghost passes and every base grid
+# k_mg_cycle
+BYTES = {
+    "ni4_amr3": (lambda: w.small_periodic(2, 4, 3, 1), PER, 3714264, 2691288),
+    "ni8_amr3": (lambda: w.small_periodic(2, 8, 3, 1), PER, 16088280, 11609304),
+    "ni16_amr3": (lambda: w.small_periodic(2, 16, 3, 4), PER, 89927248, 65292880),
+    "ni32_amr2": (lambda: w.small_periodic(2, 32, 2, 0), PER, 87937936, 64164752),
+    "ni8_amr3_isolated": (lambda: w.small_sphere(2, 8, 3, 2), SPH, 21651936, 15845856),
+    "ni8_cylinder": (lambda: w.zperiodic_cylinder(2, 8, 3), CYL, 15748040, 11600840),
+    "ni8_zmirror": (lambda: w.mirror_sphere(3, 8, 3), ZM, 12500816, 9784400),
+    "uniform64": (lambda: w.uniform_periodic(8, 8), PER, 38202696, 27585864),
+    "base5_ni4": (lambda: w.uniform_periodic(5, 4), PER, 2112616, 1520616),
+    "one_block_ni4": (lambda: w.uniform_periodic(1, 4), PER, 21448, 16712),
+    "one_block_ni16": (lambda: w.uniform_periodic(1, 16), PER, 422344, 308296),
+}
+
+
+@pytest.mark.parametrize("name", list(BYTES))
+def test_planes_cost_no_device_memory(name):
+    """The planes take the place of arrays that only the ghost passes or
+    k_mg_cycle read: a context is no larger with them, so that what fitted a
+    device before still does."""
+    mk, bc, fp64, mixed = BYTES[name]
+    h = mk()
+    for prec, most in ((abi.SFM_PREC_FP64, fp64), (abi.SFM_PREC_MIXED, mixed)):
+        with FMGPoisson(h, params=abi.default_params(bc, precision=prec, zero_mean=int(bc == PER))) as s:
+            assert s.info()["device_bytes"] <= most
+
+
 def test_solve_after_stage_dump_is_unchanged():
     """Stage dumps complete arrays a solve leaves unread; a solve on the same
     context before and after one gives the same bits."""
