@@ -228,6 +228,8 @@ extern "C" int sfm_link_blocks(int32_t nblocks, int32_t nlev, const int32_t *d_l
     k_link_check<<<ctas(nblocks), 256, 0, s>>>(nblocks, d_child, err);
     const cudaError_t launched = cudaGetLastError();
     cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (launched != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return SFM_ECUDA;
+    // the wait comes first: what was queued still writes the error word and the caller's arrays
+    const cudaError_t ran = cudaStreamSynchronize(s);
+    if (launched != cudaSuccess || ran != cudaSuccess) return SFM_ECUDA;
     return herr == 0 ? SFM_OK : SFM_EHIER;
 }
