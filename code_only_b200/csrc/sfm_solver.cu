@@ -280,6 +280,9 @@ struct Field {     // one element type, one fmg level, all blocks
     void *p = nullptr; int n = 0, G = 0; int64_t V = 0;
 };
 
+// a stage dump of the arrays as a solve leaves them (sfm_debug_solve)
+constexpr int kStageAsSolved = 16;
+
 class SolverBase {
 public:
     virtual ~SolverBase() {}
@@ -495,17 +498,17 @@ public:
     void outer_iteration_body() {
         nvtxRangePushA("sfm outer iteration");
         profNext = 0;
-        if (outerPlanes && !wholeArrays) {
-            outer_resid_planes();
-            fmg_lin();
-            outer_add_planes();
-        } else {
-            resid<double, double, T>(0, RHO[0], PSI0, SRC0, false);
-            fmg_lin();
-            add(0, PSI0, U[0]);
-        }
+        outer_resid();
+        fmg_lin();
+        if (outer_by_planes()) outer_add_planes();
+        else add(0, PSI0, U[0]);
         profPairs = profNext;
         nvtxRangePop();
+    }
+    bool outer_by_planes() const { return outerPlanes && !wholeArrays; }
+    void outer_resid() {
+        if (outer_by_planes()) outer_resid_planes();
+        else resid<double, double, T>(0, RHO[0], PSI0, SRC0, false);
     }
     template <class F>
     void with_outer_edge(F &&go) {
@@ -2334,8 +2337,10 @@ public:
     }
 
     // fmg_cycle (fmg.F90:134-233) on device arrays
-    int solve(const double *rho, double *psi, double *g, sfm_stats *stats, cudaStream_t s, int stop_stage,
+    int solve(const double *rho, double *psi, double *g, sfm_stats *stats, cudaStream_t s, int stage,
               double *dump) override {
+        const int stop_stage = stage & ~kStageAsSolved;
+        const bool whole = stage != 0 && stop_stage == stage;
         st_ = s ? s : own_;   // all work of this call is ordered on the caller's stream
         launches = 0;
         prof_init();
@@ -2345,8 +2350,8 @@ public:
         for (auto &z : zeroList) cudaMemsetAsync(z.first, 0, z.second, st_);
         cudaMemsetAsync(d_bad, 0, sizeof(int), st_);
         FmgLevel_fill0 = Undef;
-        if (wholeArrays != (stop_stage != 0)) {   // the iteration's graph was captured for the other
-            wholeArrays = stop_stage != 0;
+        if (wholeArrays != whole) {   // the iteration's graph was captured for the other
+            wholeArrays = whole;
             drop_graph();
         }
         // fmg_make_physvar
@@ -2398,10 +2403,10 @@ public:
         if (std::fabs(resh2max) <= std::numeric_limits<double>::min()) nmax = 0;
         bool conv = true, reached = (nmax == 0);
         int iters = 0;
-        if (outerPlanes && !wholeArrays && nmax > 0) outer_planes_of();
+        if (outer_by_planes() && nmax > 0) outer_planes_of();
         for (int it = 1; it <= nmax; it++) {
             if (stop_stage == 2 || stop_stage == 3) {
-                resid<double, double, T>(0, RHO[0], PSI0, SRC0, false);
+                outer_resid();
                 if (stop_stage == 2) { rc = check("resid"); return rc ? rc : dumpT(RHO[0], dump); }
                 fmg_lin();
                 rc = check("fmg_lin");
@@ -3220,7 +3225,9 @@ int sfm_debug_smoother_threads(const sfm_ctx *c, int f, int fused) {
 // Test hook (not part of include/sfmg.h): like sfm_solve on host arrays, but
 // stops after stage `stop_stage` (1 set-up, 2 first outer residual, 3 first
 // fmg_lin, 4 outer loop) and copies that stage's level-0 field, ghost width 1,
-// into `dump`.
+// into `dump`: whole arrays as the reference leaves them, or with 16 added to
+// the stage what the kernels of a solve leave, where only the cells of the
+// leaves (and at stage 1 those of refined blocks) are the reference's.
 int sfm_debug_solve(sfm_ctx *c, const double *rho, double *psi, double *g, sfm_stats *st, int stop_stage,
                     double *dump) {
     if (!c || !c->s || !rho) return SFM_EINVAL;

@@ -95,6 +95,39 @@ def test_fp64_stages_match_oracle(stage):
     assert np.array_equal(d1, d2)
 
 
+STAGE_CASES = {
+    "planes": (lambda: w.small_periodic(2, 8, 3, 5), w.gaussian_peak, abi.SFM_BC_PERIODIC),
+    "planes_ni16": (lambda: w.small_periodic(3, 16, 2, 2), w.gaussian_peak, abi.SFM_BC_PERIODIC),
+    "planes_ni4": (lambda: w.small_periodic(3, 4, 3, 2), w.gaussian_peak, abi.SFM_BC_PERIODIC),
+    "isolated": (lambda: w.small_sphere(2, 8, 3, 2), w.softened_sphere, abi.SFM_BC_SPHERE),
+    "zmirror": (lambda: w.mirror_sphere(3, 8, 3), w.wide_sphere, abi.SFM_BC_ZMIRROR),
+}
+
+
+@pytest.mark.parametrize("stage", [1, 2, 3, 4])
+@pytest.mark.parametrize("name", list(STAGE_CASES))
+def test_fp64_stages_as_solved_match_oracle(name, stage):
+    """The stages by the kernels that a solve runs (the set-up and the outer
+    iteration differ from those of a whole-array dump): every leaf cell is
+    the oracle's."""
+    mk, fn, bc = STAGE_CASES[name]
+    h = mk()
+    p = abi.default_params(bc, zero_mean=int(bc == abi.SFM_BC_PERIODIC))
+    rho = w.block_field(h, p.ngh_io, fn)
+    _, _, _, _, d1 = oracle_solve(h, rho, p, stage=stage)
+    lib = abi.load_library()
+    lib.sfm_debug_solve.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(abi.SfmStats),
+                                    C.c_int, C.c_void_p]
+    with FMGPoisson(h, params=p) as s:
+        d2 = np.zeros_like(d1)
+        psi = np.zeros_like(rho)
+        assert lib.sfm_debug_solve(s.ctx, rho.ctypes.data, psi.ctypes.data, None, None, 16 + stage, d2.ctypes.data) == 0
+    leaf = (h.child < 0).all(axis=1)
+    assert np.array_equal(interior(h, d1, 1)[leaf], interior(h, d2, 1)[leaf])
+    if stage == 1:
+        assert np.array_equal(interior(h, d1, 1), interior(h, d2, 1))
+
+
 def test_warm_start_matches_oracle():
     h = w.small_periodic(2, 8, 3, 6)
     p = abi.default_params(abi.SFM_BC_PERIODIC)

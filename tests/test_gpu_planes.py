@@ -127,7 +127,8 @@ def test_planes_cost_no_device_memory(name):
             assert s.info()["device_bytes"] <= most
 
 
-def test_solve_after_stage_dump_is_unchanged():
+@pytest.mark.parametrize("stage", [4, 16 + 4], ids=["whole_arrays", "as_solved"])
+def test_solve_after_stage_dump_is_unchanged(stage):
     """Stage dumps complete arrays a solve leaves unread; a solve on the same
     context before and after one gives the same bits."""
     h = w.small_periodic(3, 8, 3, 1)
@@ -139,7 +140,8 @@ def test_solve_after_stage_dump_is_unchanged():
     with FMGPoisson(h, params=p) as s:
         psi, g, _ = s.solve(rho)
         dump, start = np.zeros((h.nblocks,) + (h.ni + 2,) * 3), np.zeros_like(rho)
-        assert lib.sfm_debug_solve(s.ctx, rho.ctypes.data, start.ctypes.data, None, None, 4, dump.ctypes.data) == 0
+        assert lib.sfm_debug_solve(s.ctx, rho.ctypes.data, start.ctypes.data, None, None, stage,
+                                   dump.ctypes.data) == 0
         psi2, g2, _ = s.solve(rho)
     assert np.array_equal(psi, psi2) and np.array_equal(g, g2)
 
