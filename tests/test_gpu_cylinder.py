@@ -14,6 +14,7 @@ import pytest
 from code_only_b200 import abi, workloads as w
 from code_only_b200.solver import FMGPoisson, SFMError
 from tests.oracle_lib import oracle_solve
+from tests.test_gpu_planes import box
 
 pytestmark = pytest.mark.gpu
 
@@ -56,12 +57,21 @@ def test_cylinder_fp64_bitwise(oracle_runs, name):
     assert np.array_equal(g2[:, :, 2:2 + n, 2:2 + n, 2:2 + n], g1[:, :, 2:2 + n, 2:2 + n, 2:2 + n])
 
 
-@pytest.mark.parametrize("nct", [4, 16])
-def test_cylinder_base_grid_cluster_bitwise(oracle_runs, nct):
-    _, bc, mask = CASES["cyl_base8"]
-    h, rho, (rc, psi1, _, st1, _) = oracle_runs["cyl_base8"]
-    with FMGPoisson(h, params=params(bc, mask)) as s:
-        s.load_tune_table(f"base_ctas 8 16 -1 -1 {nct}\nbase_wide 8 16 -1 -1 16\n")
+@pytest.fixture(scope="module")
+def base64_run():
+    h = box(32, 4, abi.SFM_BC_CYL_ZPERIODIC)
+    rho = w.block_field(h, 2, w.beaded_line)
+    p = params(abi.SFM_BC_CYL_ZPERIODIC, 0.0)
+    p.max_outer = 2
+    return h, rho, p, oracle_solve(h, rho, p)
+
+
+@pytest.mark.parametrize("nct,wide", [(1, 16), (4, 16), (16, 16), (16, 32), (8, 64)])
+def test_cylinder_base_grid_cluster_bitwise(base64_run, nct, wide):
+    """A 64^3 base grid (k_mg_cycle), on one CTA and as a cluster"""
+    h, rho, p, (_, psi1, _, st1, _) = base64_run
+    with FMGPoisson(h, params=p) as s:
+        s.load_tune_table(f"base_ctas 8 64 -1 -1 {nct}\nbase_wide 8 64 -1 -1 {wide}\n")
         psi2, _, st2 = s.solve(rho)
     assert st2.outer_iters == st1.outer_iters
     assert np.array_equal(psi2[:, 1:-1, 1:-1, 1:-1], psi1[:, 1:-1, 1:-1, 1:-1])

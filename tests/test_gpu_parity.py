@@ -257,8 +257,16 @@ def test_solve_device_rejects_host_pointers():
         assert st.outer_iters > 0 and torch.cuda.current_device() == dev
 
 
-def test_bounded_smoother_wait_reports_timeout():
-    """Every mbarrier wait of the bulk-copy smoother is bounded.  With the
+# boxes of the smoother with planes (k_relax_faces) and with ghost passes (k_relax_bulk)
+SMOOTHER_BOXES = {
+    "planes": (lambda: w.small_periodic(2, 8, 2, 0), w.gaussian_peak, abi.SFM_BC_PERIODIC),
+    "passes": (lambda: w.mirror_sphere(2, 8, 2), w.wide_sphere, abi.SFM_BC_ZMIRROR),
+}
+
+
+@pytest.mark.parametrize("name", list(SMOOTHER_BOXES))
+def test_bounded_smoother_wait_reports_timeout(name):
+    """Every mbarrier wait of the bulk-copy smoothers is bounded.  With the
     consumers' poll limit set to zero every stage wait gives up at once: the
     CTA drains the copies it issued (their own wait keeps its full limit),
     sets the error flag and leaves, and the solve returns SFM_ETIMEOUT instead
@@ -267,22 +275,24 @@ def test_bounded_smoother_wait_reports_timeout():
     lib = abi.load_library()
     lib.sfm_debug_set_wait_polls.argtypes = [C.c_void_p, C.c_uint32]
     lib.sfm_debug_set_wait_polls.restype = C.c_int
-    h = w.small_periodic(2, 8, 2, 0)
-    p = abi.default_params(abi.SFM_BC_PERIODIC, max_outer=1)
-    rho = w.block_field(h, p.ngh_io, w.gaussian_peak)
+    mk, fn, bc = SMOOTHER_BOXES[name]
+    h, zm = mk(), int(bc == abi.SFM_BC_PERIODIC)
+    p = abi.default_params(bc, zero_mean=zm, max_outer=1)
+    rho = w.block_field(h, p.ngh_io, fn)
     with FMGPoisson(h, params=p) as s:
         assert lib.sfm_debug_set_wait_polls(s.ctx, 0) == abi.SFM_OK
         psi = np.zeros_like(rho)
         rc = lib.sfm_solve(s.ctx, rho.ctypes.data, psi.ctypes.data, None, None)
         assert rc == abi.SFM_ETIMEOUT
-    p = abi.default_params(abi.SFM_BC_PERIODIC)
+    p = abi.default_params(bc, zero_mean=zm)
     rc1, psi1, g1, st1, _ = oracle_solve(h, rho, p)
     with FMGPoisson(h, params=p) as s:
         psi2, g2, st2 = s.solve(rho)
     assert rel(psi2, psi1) == 0.0 and rel(interior(h, g2, 2), interior(h, g1, 2)) == 0.0
 
 
-def test_bounded_wait_of_the_fused_sweep_reports_timeout():
+@pytest.mark.parametrize("name", list(SMOOTHER_BOXES))
+def test_bounded_wait_of_the_fused_sweep_reports_timeout(name):
     """The same give-up in the fused sweep of the mixed path (both colours
     per launch, one barrier of the consumer warps per tile): a warp whose
     stage wait failed still reaches the tile's barrier, the barrier's OR
@@ -291,16 +301,17 @@ def test_bounded_wait_of_the_fused_sweep_reports_timeout():
     lib = abi.load_library()
     lib.sfm_debug_set_wait_polls.argtypes = [C.c_void_p, C.c_uint32]
     lib.sfm_debug_set_wait_polls.restype = C.c_int
-    h = w.small_periodic(2, 8, 2, 0)
-    p = abi.default_params(abi.SFM_BC_PERIODIC, max_outer=1, precision=abi.SFM_PREC_MIXED)
-    rho = w.block_field(h, p.ngh_io, w.gaussian_peak)
+    mk, fn, bc = SMOOTHER_BOXES[name]
+    h, zm = mk(), int(bc == abi.SFM_BC_PERIODIC)
+    p = abi.default_params(bc, zero_mean=zm, max_outer=1, precision=abi.SFM_PREC_MIXED)
+    rho = w.block_field(h, p.ngh_io, fn)
     with FMGPoisson(h, params=p) as s:
         s.load_tune_table(f"fused_sweeps 4 {h.ni} -1 -1 1\n")
         assert lib.sfm_debug_set_wait_polls(s.ctx, 0) == abi.SFM_OK
         psi = np.zeros_like(rho)
         rc = lib.sfm_solve(s.ctx, rho.ctypes.data, psi.ctypes.data, None, None)
         assert rc == abi.SFM_ETIMEOUT
-    p = abi.default_params(abi.SFM_BC_PERIODIC, rel_tol=1e-10, max_outer=40, precision=abi.SFM_PREC_MIXED)
+    p = abi.default_params(bc, zero_mean=zm, rel_tol=1e-10, max_outer=40, precision=abi.SFM_PREC_MIXED)
     with FMGPoisson(h, params=p) as s:
         s.load_tune_table(f"fused_sweeps 4 {h.ni} -1 -1 1\n")
         _, _, st = s.solve(rho)

@@ -81,8 +81,16 @@ def test_tuned_mixed_schedule_keeps_the_fp64_solution(name):
     assert np.abs(ga - gb).max() / np.abs(gb).max() <= 1e-9
 
 
+# with planes, and with ghost passes (k_relax_bulk)
+FUSED_CASES = CASES | {
+    "amr3_zmirror": (lambda: w.mirror_sphere(3, 8, 3), w.wide_sphere, abi.SFM_BC_ZMIRROR, {"zero_mean": 0}),
+    "amr2_zmirror_ni16": (lambda: w.mirror_sphere(2, 16, 2), w.wide_sphere, abi.SFM_BC_ZMIRROR, {"zero_mean": 0}),
+    "face_nested": (lambda: face_nested(8), w.gaussian_peak, abi.SFM_BC_PERIODIC, {}),
+}
+
+
 @pytest.mark.parametrize("mask,local", [(1, 1), (2, 1), (3, 1), (1, 2), (3, 2), (3, 3)])
-@pytest.mark.parametrize("name", list(CASES))
+@pytest.mark.parametrize("name", list(FUSED_CASES))
 def test_fused_sweep_keeps_the_fp64_solution(name, mask, local):
     """fused_sweeps bit 0 makes every smoothing sweep of the mixed path's
     FP32 fmg_lin one launch for both colours (the second colour with the
@@ -92,7 +100,7 @@ def test_fused_sweep_keeps_the_fp64_solution(name, mask, local):
     FP64 oracle's potential within 1e-9 at relative residual <= 1e-10, the
     profiled launches must report two colours each, and a solve after the
     table is cleared runs the two-launch sweep again (one colour each)."""
-    mk, fn, bc, kw = CASES[name]
+    mk, fn, bc, kw = FUSED_CASES[name]
     h = mk()
     p = abi.default_params(bc, rel_tol=1e-10, max_outer=40, precision=abi.SFM_PREC_MIXED, profile=1, **kw)
     rho = w.block_field(h, p.ngh_io, fn)
@@ -116,7 +124,7 @@ def test_fused_sweep_keeps_the_fp64_solution(name, mask, local):
     assert np.abs(ga - gb).max() / np.abs(gb).max() <= 1e-9
 
 
-@pytest.mark.parametrize("nt", [288, 512, 544])
+@pytest.mark.parametrize("nt", [256, 288, 512, 544])
 @pytest.mark.parametrize("name", ["amr3_periodic", "amr3_periodic_ni16"])
 def test_smoother_cta_sizes_are_bitwise(name, nt):
     """Every CTA size of the bulk-copy smoother (warp 0 producing, 7, 8, 15
@@ -216,28 +224,60 @@ def test_fp64_context_keeps_the_reference_schedule():
     assert np.array_equal(psi2[:, 1:-1, 1:-1, 1:-1], psi1[:, 1:-1, 1:-1, 1:-1])
 
 
-BASE_CASES = {
-    "uniform128": (lambda: w.uniform_periodic(16, 8), 32),   # 32^3 base grid
-    "amr_base16": (lambda: w.small_periodic(16, 8, 2, 3), 32),
-    "uniform64": (lambda: w.uniform_periodic(8, 8), 16),     # 16^3 base grid
+@pytest.fixture(scope="module")
+def base64():
+    """64^3 base grids (32^3 blocks of 4^3 cells), which k_mg_cycle serves"""
+    out = {}
+    for bc, fn in ((abi.SFM_BC_PERIODIC, w.gaussian_peak), (abi.SFM_BC_SPHERE, w.softened_sphere)):
+        h = box(32, 4, bc)
+        p = abi.default_params(bc, rel_tol=1e-10, max_outer=2, zero_mean=int(bc == abi.SFM_BC_PERIODIC))
+        rho = w.block_field(h, p.ngh_io, fn)
+        out[bc] = h, p, rho, oracle_solve(h, rho, p)
+    return out
+
+
+@pytest.mark.parametrize("nct,wide", [(1, 16), (2, 16), (4, 16), (8, 16), (8, 32), (16, 16), (16, 32), (4, 32), (4, 64),
+                                      (16, 64)])
+@pytest.mark.parametrize("bc", [abi.SFM_BC_PERIODIC, abi.SFM_BC_SPHERE], ids=["periodic", "isolated"])
+def test_base_grid_cluster_is_bitwise(base64, bc, nct, wide):
+    """k_mg_cycle as a cluster of CTAs (the large levels spread over every
+    CTA, the small ones on CTA 0, the maxima over the cluster) computes every
+    cell with the same expression: the FP64 solve stays bit-identical to the
+    oracle whatever the shape.  A shape the GPU cannot hold resident falls
+    back to one CTA, which must match as well."""
+    h, p, rho, (_, psi_o, g_o, st_o, _) = base64[bc]
+    with FMGPoisson(h, params=p) as s:
+        s.load_tune_table(f"base_ctas 8 64 -1 -1 {nct}\nbase_wide 8 64 -1 -1 {wide}\n")
+        psi, g, st = s.solve(rho)
+        psi2, g2, _ = s.solve(rho)                       # the graph replayed
+    assert st.outer_iters == st_o.outer_iters
+    assert np.array_equal(psi[:, 1:-1, 1:-1, 1:-1], psi_o[:, 1:-1, 1:-1, 1:-1])
+    n = h.ni
+    assert np.array_equal(g[:, :, 2:2 + n, 2:2 + n, 2:2 + n], g_o[:, :, 2:2 + n, 2:2 + n, 2:2 + n])
+    assert np.array_equal(psi, psi2) and np.array_equal(g, g2)
+
+
+# base grids that k_mgs_cycle serves, and a shape of k_mg_cycle for each
+SMALL_BASE_CASES = {
+    "uniform128": (lambda: w.uniform_periodic(16, 8), 32, 16, 16),
+    "amr_base16": (lambda: w.small_periodic(16, 8, 2, 3), 32, 4, 32),
+    "uniform64": (lambda: w.uniform_periodic(8, 8), 16, 8, 16),
 }
 
 
-@pytest.mark.parametrize("nct,wide", [(2, 16), (4, 16), (8, 16), (8, 32), (16, 16), (4, 32)])
-@pytest.mark.parametrize("name", list(BASE_CASES))
-def test_base_grid_cluster_is_bitwise(name, nct, wide):
-    """The base-grid multigrid as a cluster of CTAs (the large levels spread
-    over every CTA, the small ones on CTA 0, the maxima over the cluster)
-    computes every cell with the same expression: the FP64 solve stays
-    bit-identical to the oracle whatever the shape.  A shape the GPU cannot
-    hold resident falls back to one CTA, which must match as well."""
-    mk, nbase = BASE_CASES[name]
+@pytest.mark.parametrize("name", list(SMALL_BASE_CASES))
+def test_base_grid_rows_of_an_old_table_are_accepted(name):
+    """Up to 32^3 cells the base grid has one launch shape: rows for it in a
+    saved table load, and the FP64 solve is the oracle's."""
+    mk, nbase, nct, wide = SMALL_BASE_CASES[name]
     h = mk()
     p = abi.default_params(abi.SFM_BC_PERIODIC, rel_tol=1e-10, max_outer=30)
     rho = w.block_field(h, p.ngh_io, w.gaussian_peak)
     _, psi_o, g_o, st_o, _ = oracle_solve(h, rho, p)
+    table = f"base_ctas 8 {nbase} -1 -1 {nct}\nbase_wide 8 {nbase} -1 -1 {wide}\n"
     with FMGPoisson(h, params=p) as s:
-        s.load_tune_table(f"base_ctas 8 {nbase} -1 -1 {nct}\nbase_wide 8 {nbase} -1 -1 {wide}\n")
+        s.load_tune_table(table)
+        assert sorted(s.tune_table().splitlines()[1:]) == sorted(table.splitlines())
         psi, g, st = s.solve(rho)
         psi2, g2, _ = s.solve(rho)                       # the graph replayed
     assert st.outer_iters == st_o.outer_iters

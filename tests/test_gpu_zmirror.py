@@ -7,7 +7,8 @@ FP64 must be bit-identical to the oracle (psi with its ghost layer, g, the
 outer iteration count) on boxes whose base grid takes the reference's
 base-level sweeps (3^3 base blocks) and boxes whose base grid runs the
 serial multigrid with the mirror on its z-min face (2^3 and 8^3 base
-blocks; on the latter also as a thread-block cluster).  The mixed path must
+blocks; 32^3 blocks of 4^3 cells for the kernel of large base grids, on one
+CTA and as a thread-block cluster).  The mixed path must
 reach the FP64 oracle's potential within 1e-9, and the half box must give
 the potential of the mirror-symmetric full box with the ordinary isolated
 boundary."""
@@ -17,6 +18,7 @@ import pytest
 from code_only_b200 import abi, workloads as w
 from code_only_b200.solver import FMGPoisson, SFMError
 from tests.oracle_lib import oracle_solve
+from tests.test_gpu_planes import box
 
 pytestmark = pytest.mark.gpu
 
@@ -58,13 +60,22 @@ def test_zmirror_fp64_bitwise(oracle_runs, name):
     assert np.array_equal(g2[:, :, 2:2 + n, 2:2 + n, 2:2 + n], g1[:, :, 2:2 + n, 2:2 + n, 2:2 + n])
 
 
-@pytest.mark.parametrize("nct", [4, 16])
-def test_zmirror_base_grid_cluster_bitwise(oracle_runs, nct):
-    """The 16^3 base grid of the 8^3-block box as a cluster: the mirror
-    steps spread over every CTA on the large levels."""
-    h, rho, (rc, psi1, g1, st1, _) = oracle_runs["base8_l2"]
-    with FMGPoisson(h, params=params()) as s:
-        s.load_tune_table(f"base_ctas 8 16 -1 -1 {nct}\nbase_wide 8 16 -1 -1 16\n")
+@pytest.fixture(scope="module")
+def base64_run():
+    h = box(32, 4, abi.SFM_BC_ZMIRROR)
+    rho = w.block_field(h, 2, w.wide_sphere)
+    p = params()
+    p.max_outer = 2
+    return h, rho, p, oracle_solve(h, rho, p)
+
+
+@pytest.mark.parametrize("nct,wide", [(1, 16), (4, 16), (16, 16), (16, 32), (8, 64)])
+def test_zmirror_base_grid_cluster_bitwise(base64_run, nct, wide):
+    """A 64^3 base grid (k_mg_cycle) as a cluster: the mirror steps spread
+    over every CTA on the large levels."""
+    h, rho, p, (_, psi1, _, st1, _) = base64_run
+    with FMGPoisson(h, params=p) as s:
+        s.load_tune_table(f"base_ctas 8 64 -1 -1 {nct}\nbase_wide 8 64 -1 -1 {wide}\n")
         psi2, _, st2 = s.solve(rho)
     assert st2.outer_iters == st1.outer_iters
     assert np.array_equal(psi2[:, 1:-1, 1:-1, 1:-1], psi1[:, 1:-1, 1:-1, 1:-1])
