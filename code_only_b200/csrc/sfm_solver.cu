@@ -359,7 +359,8 @@ public:
     CFItem *d_cf = nullptr;
     std::vector<T *> faceBuf[2], cfBuf;
     std::vector<int> facePar;              // buffer holding U[f]'s planes, -1: neither
-    // the outer residual's (boxes without physical-boundary faces): planes of PSI0 ([6 nb][n^2], fewer values than RES0d's)
+    // the outer residual's (boxes without physical-boundary faces): planes of
+    // PSI0, [6 nb][n^2] values (fewer than RES0d's)
     double *outerPlanes = nullptr, *outerCf = nullptr;
     // whole arrays as the reference leaves them, unread ghost cells and
     // refined blocks included (the debug entry's stage dumps compare them)
@@ -3169,9 +3170,10 @@ int sfm_info(const sfm_ctx *c, int32_t *fmg_levels, int64_t *device_bytes) {
     return SFM_OK;
 }
 
-// Test hook (not part of include/sfmg.h): poll limit of the smoother's
-// consumer stage waits (k_relax_bulk); 0 makes every such wait give up at
-// once, so a solve exercises the bounded-wait error path (SFM_ETIMEOUT).
+// Test hook (not part of include/sfmg.h): poll limit of the smoothers'
+// consumer stage waits (k_relax_faces, k_relax_bulk); 0 makes every such wait
+// give up at once, so a solve exercises the bounded-wait error path
+// (SFM_ETIMEOUT).
 int sfm_debug_set_wait_polls(sfm_ctx *c, uint32_t polls) {
     if (!c || !c->s) return SFM_EINVAL;
     c->s->set_wait_polls(polls);

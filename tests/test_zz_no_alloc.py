@@ -6,7 +6,7 @@ Both converge the same 7-point periodic problem lap(phi) = 4 pi (rho - mean)
 on the same grid, so after removing the free constant they agree to the
 convergence tolerance: 1e-8 relative (max norm) with both solves run to a
 relative residual of 1e-12.  Two calls in a row must both pass, and give
-identical results (the kernel clears its fixed scratch itself).  The file
+identical results (nothing carries over between calls).  The file
 name puts it after every other GPU test; it also passes alone.
 """
 import ctypes as C
@@ -145,7 +145,7 @@ def test_noalloc_refuses_host_outputs_under_capture():
     rho = torch.ones((n, n, n), dtype=torch.float64, device="cuda")
     psi = torch.zeros_like(rho)
     s = torch.cuda.Stream()
-    # a first call outside capture looks up the scratch array
+    # a first call outside capture sets the kernels up
     assert f(rho.data_ptr(), psi.data_ptr(), n, 1.0 / n, 1.0, 1e-10, 10, None, None,
              C.c_void_p(s.cuda_stream)) == abi.SFM_OK
     torch.cuda.synchronize()
